@@ -54,6 +54,7 @@ extern "C" void qb_destroy(qb_ctx *ctx) {
     if (ctx->err_flag_dev) cudaFree(ctx->err_flag_dev);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->scratch2) cudaFree(ctx->scratch2);
+    if (ctx->scratch3) cudaFree(ctx->scratch3);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -73,33 +74,23 @@ extern "C" void *qb_stream(qb_ctx *ctx) { return (void *)ctx->stream; }
 extern "C" int qb_sm_count(qb_ctx *ctx) { return ctx->sm_count; }
 extern "C" int64_t qb_launch_count(qb_ctx *ctx) { return ctx->launches; }
 
-int qb_ctx_scratch(qb_ctx *ctx, size_t bytes, void **out) {
-    if (bytes > ctx->scratch_bytes) {
+// Grown on demand, with a quarter to spare; whatever may still use the old buffer is waited for first.
+static int grow(qb_ctx *ctx, void *&buf, size_t &have, size_t bytes, void **out) {
+    if (bytes > have) {
         QB_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (ctx->scratch) QB_CUDA(cudaFree(ctx->scratch));
-        ctx->scratch = nullptr;
-        ctx->scratch_bytes = 0;
+        if (buf) QB_CUDA(cudaFree(buf));
+        buf = nullptr;
+        have = 0;
         const size_t want = bytes + (bytes >> 2) + (1u << 20);
-        QB_CUDA(cudaMalloc(&ctx->scratch, want));
-        ctx->scratch_bytes = want;
+        QB_CUDA(cudaMalloc(&buf, want));
+        have = want;
     }
-    *out = ctx->scratch;
+    *out = buf;
     return QB_OK;
 }
-
-int qb_ctx_scratch2(qb_ctx *ctx, size_t bytes, void **out) {
-    if (bytes > ctx->scratch2_bytes) {
-        QB_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (ctx->scratch2) QB_CUDA(cudaFree(ctx->scratch2));
-        ctx->scratch2 = nullptr;
-        ctx->scratch2_bytes = 0;
-        const size_t want = bytes + (bytes >> 2) + (1u << 20);
-        QB_CUDA(cudaMalloc(&ctx->scratch2, want));
-        ctx->scratch2_bytes = want;
-    }
-    *out = ctx->scratch2;
-    return QB_OK;
-}
+int qb_ctx_scratch(qb_ctx *ctx, size_t bytes, void **out) { return grow(ctx, ctx->scratch, ctx->scratch_bytes, bytes, out); }
+int qb_ctx_scratch2(qb_ctx *ctx, size_t bytes, void **out) { return grow(ctx, ctx->scratch2, ctx->scratch2_bytes, bytes, out); }
+int qb_ctx_scratch3(qb_ctx *ctx, size_t bytes, void **out) { return grow(ctx, ctx->scratch3, ctx->scratch3_bytes, bytes, out); }
 
 extern "C" int qb_mem_info(qb_ctx *ctx, size_t *free_bytes, size_t *total_bytes) {
     QB_REQUIRE(ctx, "qb_mem_info: null context");

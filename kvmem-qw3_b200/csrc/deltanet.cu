@@ -14,12 +14,6 @@
 
 namespace {
 
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // ---- one kernel for the whole layer -------------------------------------------------------------------------
 // grid (HD/COLS, nv, n_seqs), cluster (HD/COLS, 1, 1), block 512: the CTAs of a cluster share one v head, each owns
 // COLS = 32 or 64 state columns (a warp 2 or 4 of them, lanes stripe the k dimension).  Rows are processed in blocks of 4:
@@ -31,9 +25,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 //   columns (= one quantisation block).
 // The q/k conv windows are read by several CTAs but written by one (v head < nk, column block 0), so the kernel
 // reads the conv state from conv and writes it to conv_out (a different buffer: the caller ping-pongs).
-// RB = rows per block (one conv / norm phase, one exchange of the head's sums of squares and one norm-gate phase per
-// block): 4 for the decode and verify steps, 8 for prompt ingestion, where the per-block costs dominate.  A row's
-// arithmetic does not depend on RB.
+// RB = rows per block (one conv / norm phase, one exchange of the head's sums of squares and one norm-gate phase per block).
 template <int HD, int CPW, int RB, int MINB>
 __global__ void __launch_bounds__(512, MINB) dn_fused_kernel(DnArgs a) {
     constexpr int COLS = 16 * CPW, NCB = HD / COLS, NQB = COLS / 32, RPL = HD / 32, NCH = 2 * HD + COLS;
@@ -65,67 +57,33 @@ __global__ void __launch_bounds__(512, MINB) dn_fused_kernel(DnArgs a) {
     // The inputs of a row block (projection rows, gate inputs, z) do not depend on the state slot: they are
     // requested first, and the next block's while the current one is processed.
     struct BlockIn { float cur[RB]; float zv, graw; };
-    // Ingestion form: every load of a block is issued before the first add (a load-add-load-add chain exposes one memory
-    // latency per row); each element still adds its K-segment partials in ascending order.
     auto load_block = [&](uint32_t rb0) {
         BlockIn in;
         const uint32_t nrows = rb0 < R ? min((uint32_t)RB, R - rb0) : 0u;
         const size_t row0 = (size_t)seq * R + rb0;
-        if constexpr (RB <= 4) {
-            // the step forms (64 registers per thread): element by element
-            if (a.proj_S == 2) {                      // the usual split of the input projection: both partials of every row first
-                float p1[RB];
+        if (a.proj_S == 2) {                      // the usual split of the input projection: both partials of every row first
+            float p1[RB];
 #pragma unroll
-                for (int t = 0; t < RB; ++t) {
-                    const bool on = has && (uint32_t)t < nrows;
-                    in.cur[t] = on ? a.proj[(row0 + t) * a.proj_stride + ch] : 0.0f;
-                    p1[t] = on ? a.proj[(row0 + t) * a.proj_stride + ch + a.proj_pstride] : 0.0f;
-                }
-#pragma unroll
-                for (int t = 0; t < RB; ++t) in.cur[t] += p1[t];
-            } else {
-#pragma unroll
-                for (int t = 0; t < RB; ++t) {
-                    in.cur[t] = 0.0f;
-                    if (has && (uint32_t)t < nrows) in.cur[t] = qb_ldsum(a.proj, (row0 + t) * a.proj_stride + ch, a.proj_S, a.proj_pstride);
-                }
+            for (int t = 0; t < RB; ++t) {
+                const bool on = has && (uint32_t)t < nrows;
+                in.cur[t] = on ? a.proj[(row0 + t) * a.proj_stride + ch] : 0.0f;
+                p1[t] = on ? a.proj[(row0 + t) * a.proj_stride + ch + a.proj_pstride] : 0.0f;
             }
-            in.zv = 0.0f;
-            if (ng_q < NQB && ng_t < nrows)
-                in.zv = qb_ldsum(a.proj, (row0 + ng_t) * a.proj_stride + C + vh * HD + cb * COLS + ng_q * 32 + lane, a.proj_S, a.proj_pstride);
-            in.graw = 0.0f;
-            if (warp == 15 && lane < 2 * nrows)      // (row, decay | write strength) of the block: lanes of the last warp
-                in.graw = qb_ldsum(a.proj, (row0 + (lane >> 1)) * a.proj_stride + C + vdim + (lane & 1) * a.nv + vh, a.proj_S, a.proj_pstride);
-            return in;
+#pragma unroll
+            for (int t = 0; t < RB; ++t) in.cur[t] += p1[t];
+        } else {
+#pragma unroll
+            for (int t = 0; t < RB; ++t) {
+                in.cur[t] = 0.0f;
+                if (has && (uint32_t)t < nrows) in.cur[t] = qb_ldsum(a.proj, (row0 + t) * a.proj_stride + ch, a.proj_S, a.proj_pstride);
+            }
         }
-        const uint32_t S = a.proj_S;
-        const bool two = S > 1;
-        const bool hz = ng_q < NQB && ng_t < nrows, hg = warp == 15 && lane < 2 * nrows;
-        const size_t iz = (row0 + ng_t) * a.proj_stride + C + vh * HD + cb * COLS + ng_q * 32 + lane;
-        const size_t ig = (row0 + (lane >> 1)) * a.proj_stride + C + vdim + (lane & 1) * a.nv + vh;
-        float p0[RB], p1[RB];
-#pragma unroll
-        for (int t = 0; t < RB; ++t) {
-            const bool on = has && (uint32_t)t < nrows;
-            p0[t] = on ? a.proj[(row0 + t) * a.proj_stride + ch] : 0.0f;
-            p1[t] = on && two ? a.proj[(row0 + t) * a.proj_stride + ch + a.proj_pstride] : 0.0f;
-        }
-        const float z0 = hz ? a.proj[iz] : 0.0f, z1 = hz && two ? a.proj[iz + a.proj_pstride] : 0.0f;
-        const float g0 = hg ? a.proj[ig] : 0.0f, g1 = hg && two ? a.proj[ig + a.proj_pstride] : 0.0f;
-#pragma unroll
-        for (int t = 0; t < RB; ++t) in.cur[t] = two ? p0[t] + p1[t] : p0[t];
-        in.zv = two ? z0 + z1 : z0;
-        in.graw = two ? g0 + g1 : g0;
-        for (uint32_t sg = 2; sg < S; ++sg) {                 // further segments: again all loads, then the adds
-            const size_t off = (size_t)sg * a.proj_pstride;
-#pragma unroll
-            for (int t = 0; t < RB; ++t) p0[t] = has && (uint32_t)t < nrows ? a.proj[(row0 + t) * a.proj_stride + ch + off] : 0.0f;
-            const float zs = hz ? a.proj[iz + off] : 0.0f, gs = hg ? a.proj[ig + off] : 0.0f;
-#pragma unroll
-            for (int t = 0; t < RB; ++t) in.cur[t] += p0[t];
-            in.zv += zs;
-            in.graw += gs;
-        }
+        in.zv = 0.0f;
+        if (ng_q < NQB && ng_t < nrows)
+            in.zv = qb_ldsum(a.proj, (row0 + ng_t) * a.proj_stride + C + vh * HD + cb * COLS + ng_q * 32 + lane, a.proj_S, a.proj_pstride);
+        in.graw = 0.0f;
+        if (warp == 15 && lane < 2 * nrows)      // (row, decay | write strength) of the block: lanes of the last warp
+            in.graw = qb_ldsum(a.proj, (row0 + (lane >> 1)) * a.proj_stride + C + vdim + (lane & 1) * a.nv + vh, a.proj_S, a.proj_pstride);
         return in;
     };
     BlockIn nxt = load_block(0);
@@ -398,6 +356,274 @@ int launch_fused(qb_ctx *ctx, const DnArgs &a) {
     return QB_OK;
 }
 
+// ---- prompt ingestion: three launches per layer ---------------------------------------------------------------
+// One CTA of dn_fused_kernel spends most of a row waiting: two five-step exchanges over 32 lanes, the barriers of the conv and
+// norm phases, one CTA per SM (1.16 us per row, 595 us per 512 rows and layer at 48 heads of 128).  Only the delta rule is
+// sequential, so for many rows everything else leaves that chain:
+//   dn_prep_kernel   conv + SiLU, L2 norm, gates of all rows at once
+//   dn_scan_kernel   the delta rule; a column of the state is held by 8 lanes (16 of its 128 values each at head size 128): three
+//                    exchange steps instead of five, two of them shared by the columns of a thread; rows arrive by cp.async
+//   dn_gate_kernel   head-wide RMSNorm * gain * SiLU(z), quantisation, all rows at once
+// Every sum is formed from the same pairs in the same order as in dn_fused_kernel (a lane adds the partial sums of the four lanes
+// it stands for as the first two exchange steps would), so a row has the same bits in either form.
+constexpr uint32_t DN_PB = 8;                    // rows per block of the two parallel kernels
+
+// q and k are stored so that a lane of the scan reads its values with 16-byte loads: inside every 32 values, index 8j + m is at 4m + j.
+template <int HD>
+__global__ void __launch_bounds__(HD) dn_prep_kernel(DnArgs a, float *__restrict__ qk, float *__restrict__ vc, float *__restrict__ gb) {
+    QB_PDL_ENTER();
+    __shared__ float red[DN_PB][HD / 32];
+    const uint32_t u = blockIdx.x, rb0 = blockIdx.y * DN_PB, seq = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t R = a.rows_per_seq, nrows = min(DN_PB, R - rb0), ch = u * HD + tid;
+    const uint32_t C = 2 * a.nk * HD + a.nv * HD, vdim = a.nv * HD;
+    const size_t row0 = (size_t)seq * R + rb0;
+    const bool is_qk = u < 2 * a.nk;
+    float cur[DN_PB + 3], w[4];
+    const float *src = a.proj + row0 * a.proj_stride + ch;
+    if (rb0 == 0) {
+        const float *conv_in = a.conv + ((size_t)seq * a.n_slots + (uint32_t)a.slot_in[seq]) * C * 3 + (size_t)ch * 3;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) cur[k] = conv_in[k];
+    } else {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) cur[k] = src[-(ptrdiff_t)(3 - k) * a.proj_stride];
+    }
+#pragma unroll
+    for (int t = 0; t < (int)DN_PB; ++t) cur[3 + t] = (uint32_t)t < nrows ? src[(size_t)t * a.proj_stride] : 0.0f;
+    for (uint32_t sg = 1; sg < a.proj_S; ++sg) {                // all loads of a segment, then the adds (ascending segments)
+        const float *ps = src + (size_t)sg * a.proj_pstride;
+        float p[DN_PB + 3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) p[k] = rb0 ? ps[-(ptrdiff_t)(3 - k) * a.proj_stride] : 0.0f;
+#pragma unroll
+        for (int t = 0; t < (int)DN_PB; ++t) p[3 + t] = (uint32_t)t < nrows ? ps[(size_t)t * a.proj_stride] : 0.0f;
+        if (rb0) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) cur[k] += p[k];
+        }
+#pragma unroll
+        for (int t = 0; t < (int)DN_PB; ++t) cur[3 + t] += p[3 + t];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k] = a.conv_w[(size_t)ch * 4 + k];
+    float x[DN_PB];
+#pragma unroll
+    for (int t = 0; t < (int)DN_PB; ++t) {
+        float acc = w[3] * cur[3 + t];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) acc += w[k] * cur[t + k];
+        x[t] = __fdiv_rn(acc, 1.0f + expf(-acc));
+    }
+    if (is_qk) {
+#pragma unroll
+        for (int t = 0; t < (int)DN_PB; ++t) {
+            const float ss = warp_sum(x[t] * x[t]);
+            if (lane == 0) red[t][warp] = ss;
+        }
+        __syncthreads();
+        const uint32_t head = u < a.nk ? u : u - a.nk, pos = (u < a.nk ? 0 : HD) + warp * 32 + 4 * (lane & 7) + (lane >> 3);
+        float *dst = qk + row0 * (a.nk * 2 * HD) + head * 2 * HD + pos;
+#pragma unroll
+        for (int t = 0; t < (int)DN_PB; ++t) {
+            float tot = 0.0f;
+#pragma unroll
+            for (int k = 0; k < HD / 32; ++k) tot += red[t][k];
+            if ((uint32_t)t < nrows) dst[(size_t)t * (a.nk * 2 * HD)] = x[t] * rsqrtf(tot + a.eps);
+        }
+    } else {
+        const uint32_t vh = u - 2 * a.nk;
+#pragma unroll
+        for (int t = 0; t < (int)DN_PB; ++t)
+            if ((uint32_t)t < nrows) vc[(row0 + t) * vdim + vh * HD + tid] = x[t];
+        if (tid < 2 * nrows) {                                   // (row, decay | write strength)
+            const float graw = qb_ldsum(a.proj, (row0 + (tid >> 1)) * a.proj_stride + C + vdim + (tid & 1) * a.nv + vh, a.proj_S, a.proj_pstride);
+            gb[(row0 + (tid >> 1)) * (2 * a.nv) + 2 * vh + (tid & 1)] =
+                (tid & 1) == 0 ? expf(log1pf(expf(graw + a.dt_bias[vh])) * a.ssm_a[vh]) : __fdiv_rn(1.0f, 1.0f + expf(-graw));
+        }
+    }
+    if (rb0 + nrows == R) {                                      // the new window: the last three inputs
+        float *conv_out = a.conv_out + (size_t)seq * a.n_slots * C * 3 + (size_t)ch * 3;
+#pragma unroll
+        for (int t = 0; t < (int)DN_PB; ++t)
+            if ((uint32_t)t + 1 == nrows) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) conv_out[k] = cur[t + 1 + k];
+            }
+    }
+}
+
+// grid (HD / COLS, nv, n_seqs): a CTA owns COLS = NW * 4 * CPT state columns of a head, a thread 1/8 of CPT columns.  The core
+// output takes the place of v in vc (a CTA has read a row's v before it writes that row).
+template <int HD, int CPT, int NW>
+__global__ void __launch_bounds__(32 * NW) dn_scan_kernel(DnArgs a, const float *__restrict__ qk, float *vc, const float *__restrict__ gb) {
+    QB_PDL_ENTER();
+    constexpr int COLS = NW * 4 * CPT, NR = HD / 32, TR = 16, PITCH = 2 * HD + COLS + 4;
+    static_assert(CPT == 2 || CPT == 4, "columns per thread");
+    __shared__ __align__(16) float buf[2][TR][PITCH];
+    const uint32_t vh = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t m = lane & 7, lc = warp * 4 * CPT + (lane >> 3) * CPT, kh = vh % a.nk, R = a.rows_per_seq, vdim = a.nv * HD;
+    const size_t row0 = (size_t)seq * R, ssz = (size_t)a.nv * HD * HD;
+    const float *qk_src = qk + row0 * (a.nk * 2 * HD) + kh * 2 * HD;
+    float *v_src = vc + row0 * vdim + vh * HD + blockIdx.x * COLS;
+    const float *gb_src = gb + row0 * (2 * a.nv) + 2 * vh;
+    auto fetch = [&](uint32_t t0, uint32_t bf) {
+        constexpr int Q4 = 2 * HD / 4, V4 = COLS / 4, PER = Q4 + V4 + 1;
+        const uint32_t n = t0 < R ? min((uint32_t)TR, R - t0) * PER : 0u;
+        for (uint32_t i = tid; i < n; i += 32 * NW) {
+            const uint32_t t = i / PER, p = i % PER;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&buf[bf][t][0]);
+            if (p < Q4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + p * 16), "l"(qk_src + (size_t)(t0 + t) * (a.nk * 2 * HD) + p * 4) : "memory");
+            else if (p < Q4 + V4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + p * 16), "l"(v_src + (size_t)(t0 + t) * vdim + (p - Q4) * 4) : "memory");
+            else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + p * 16), "l"(gb_src + (size_t)(t0 + t) * (2 * a.nv)) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, 0);
+    float s[CPT][NR][4];
+    const float *st_in = a.state + ((size_t)seq * a.n_slots + (uint32_t)a.slot_in[seq]) * ssz + ((size_t)vh * HD + blockIdx.x * COLS + lc) * HD + m;
+#pragma unroll
+    for (int c = 0; c < CPT; ++c)
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[c][r][j] = st_in[(size_t)c * HD + r * 32 + 8 * j];
+    const float oscale = rsqrtf((float)HD);
+    const bool hi4 = (m & 4) != 0, hi2 = (m & 2) != 0;
+    // Totals over a column's 8 lanes: the first step (CPT 4: the first two) halves the columns a lane carries.  The lane ends with the
+    // total of column 2 * hi4 + hi2 (CPT 4) or hi4 (CPT 2).
+    auto total = [&](const float (&v)[CPT]) -> float {
+        float k;
+        if constexpr (CPT == 4) {
+            float k0 = hi4 ? v[2] : v[0], k1 = hi4 ? v[3] : v[1];
+            const float s0 = hi4 ? v[0] : v[2], s1 = hi4 ? v[1] : v[3];
+            k0 += __shfl_xor_sync(0xffffffffu, s0, 4);
+            k1 += __shfl_xor_sync(0xffffffffu, s1, 4);
+            k = hi2 ? k1 : k0;
+            const float sd = hi2 ? k0 : k1;
+            k += __shfl_xor_sync(0xffffffffu, sd, 2);
+        } else {
+            k = hi4 ? v[1] : v[0];
+            const float sd = hi4 ? v[0] : v[1];
+            k += __shfl_xor_sync(0xffffffffu, sd, 4);
+            k += __shfl_xor_sync(0xffffffffu, k, 2);
+        }
+        return k + __shfl_xor_sync(0xffffffffu, k, 1);
+    };
+    for (uint32_t t0 = 0, bf = 0; t0 < R; t0 += TR, bf ^= 1) {
+        fetch(t0 + TR, bf ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const uint32_t n = min((uint32_t)TR, R - t0);
+#pragma unroll 2
+        for (uint32_t t = 0; t < n; ++t) {
+            const float *row = buf[bf][t];
+            const float g = row[2 * HD + COLS], beta = row[2 * HD + COLS + 1];
+            float4 kr[NR], qr[NR];
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                kr[r] = *reinterpret_cast<const float4 *>(row + HD + r * 32 + 4 * m);
+                qr[r] = *reinterpret_cast<const float4 *>(row + r * 32 + 4 * m);
+            }
+            float part[CPT];
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) {
+                float p[4] = {0.0f, 0.0f, 0.0f, 0.0f};          // the four lanes this one stands for: m, m + 8, m + 16, m + 24
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    p[0] += s[c][r][0] * kr[r].x; p[1] += s[c][r][1] * kr[r].y; p[2] += s[c][r][2] * kr[r].z; p[3] += s[c][r][3] * kr[r].w;
+                }
+                part[c] = (p[0] + p[2]) + (p[1] + p[3]);
+            }
+            const float kvt = total(part);
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) {
+                const float kv = __shfl_sync(0xffffffffu, kvt, CPT == 4 ? 4 * (c >> 1) + 2 * (c & 1) : 4 * c, 8);
+                const float delta = (row[2 * HD + lc + c] - g * kv) * beta;
+                float p[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    s[c][r][0] = g * s[c][r][0] + kr[r].x * delta; p[0] += s[c][r][0] * qr[r].x;
+                    s[c][r][1] = g * s[c][r][1] + kr[r].y * delta; p[1] += s[c][r][1] * qr[r].y;
+                    s[c][r][2] = g * s[c][r][2] + kr[r].z * delta; p[2] += s[c][r][2] * qr[r].z;
+                    s[c][r][3] = g * s[c][r][3] + kr[r].w * delta; p[3] += s[c][r][3] * qr[r].w;
+                }
+                part[c] = (p[0] + p[2]) + (p[1] + p[3]);
+            }
+            const float att = total(part);
+            if (CPT == 4 ? (m & 1) == 0 : (m & 3) == 0) v_src[(size_t)(t0 + t) * vdim + lc + (CPT == 4 ? m >> 1 : m >> 2)] = att * oscale;
+        }
+        __syncthreads();                                         // the buffer is free for the fetch of the next round
+    }
+    float *st_out = a.state + (size_t)seq * a.n_slots * ssz + ((size_t)vh * HD + blockIdx.x * COLS + lc) * HD + m;
+#pragma unroll
+    for (int c = 0; c < CPT; ++c)
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) st_out[(size_t)c * HD + r * 32 + 8 * j] = s[c][r][j];
+}
+
+template <int HD>
+__global__ void __launch_bounds__(HD) dn_gate_kernel(DnArgs a, const float *__restrict__ core) {
+    QB_PDL_ENTER();
+    __shared__ float red[DN_PB][HD / 32];
+    const uint32_t vh = blockIdx.x, seq = blockIdx.z, rb0 = blockIdx.y * DN_PB, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t R = a.rows_per_seq, nrows = min(DN_PB, R - rb0), C = 2 * a.nk * HD + a.nv * HD, vdim = a.nv * HD, col = vh * HD + tid;
+    const size_t row0 = (size_t)seq * R + rb0;
+    float v[DN_PB], z[DN_PB];
+#pragma unroll
+    for (int t = 0; t < (int)DN_PB; ++t) {
+        v[t] = (uint32_t)t < nrows ? core[(row0 + t) * vdim + col] : 0.0f;
+        z[t] = (uint32_t)t < nrows ? a.proj[(row0 + t) * a.proj_stride + C + col] : 0.0f;
+    }
+    for (uint32_t sg = 1; sg < a.proj_S; ++sg) {
+        float p[DN_PB];
+#pragma unroll
+        for (int t = 0; t < (int)DN_PB; ++t) p[t] = (uint32_t)t < nrows ? a.proj[(row0 + t) * a.proj_stride + C + col + sg * a.proj_pstride] : 0.0f;
+#pragma unroll
+        for (int t = 0; t < (int)DN_PB; ++t) z[t] += p[t];
+    }
+    const float nw = a.norm_w[tid];
+#pragma unroll
+    for (int t = 0; t < (int)DN_PB; ++t) {
+        const float ss = warp_sum(v[t] * v[t]);
+        if (lane == 0) red[t][warp] = ss;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < (int)DN_PB; ++t) {
+        if ((uint32_t)t >= nrows) break;
+        float tot = 0.0f;
+#pragma unroll
+        for (int r = 0; r < HD / 32; ++r) tot += red[t][r];
+        const float o = v[t] * rsqrtf(tot / (float)HD + a.eps) * nw * __fdiv_rn(z[t], 1.0f + expf(-z[t]));
+        const size_t row = row0 + t;
+        if (a.core_out) a.core_out[row * vdim + col] = o;
+        if (a.q8) quant_block_store(o, (int)lane, a.q8 + row * a.q_pitch + (col & ~31u), a.d + (size_t)(col / 32) * a.d_ld + row);
+    }
+}
+
+template <int HD>
+int launch_ingest(qb_ctx *ctx, const DnArgs &a) {
+    constexpr int CPT = 4, NW = HD == 128 ? 4 : 2;               // 64 (32) columns per CTA
+    const size_t rows = (size_t)a.n_seqs * a.rows_per_seq, nqk = rows * a.nk * 2 * HD, nvc = rows * a.nv * HD, need = nqk + nvc + rows * 2 * a.nv;
+    float *work = a.work;
+    if (!work || need > a.work_floats) {
+        void *p = nullptr;
+        QB_TRY(qb_ctx_scratch3(ctx, need * sizeof(float), &p));
+        work = (float *)p;
+    }
+    float *qk = work, *vc = work + nqk, *gb = vc + nvc;
+    const uint32_t rblk = (a.rows_per_seq + DN_PB - 1) / DN_PB;
+    QB_CUDA(qb_launch_pdl(ctx->stream, dn_prep_kernel<HD>, dim3(2 * a.nk + a.nv, rblk, a.n_seqs), dim3(HD), 0, a, qk, vc, gb));
+    QB_LAUNCHED(ctx, "dn_prep_kernel");
+    QB_CUDA(qb_launch_pdl(ctx->stream, dn_scan_kernel<HD, CPT, NW>, dim3(HD / (NW * 4 * CPT), a.nv, a.n_seqs), dim3(32 * NW), 0, a, (const float *)qk, vc, (const float *)gb));
+    QB_LAUNCHED(ctx, "dn_scan_kernel");
+    QB_CUDA(qb_launch_pdl(ctx->stream, dn_gate_kernel<HD>, dim3(a.nv, rblk, a.n_seqs), dim3(HD), 0, a, (const float *)vc));
+    QB_LAUNCHED(ctx, "dn_gate_kernel");
+    return QB_OK;
+}
+
 }  // namespace
 
 int qb_launch_deltanet(qb_ctx *ctx, const DnArgs &a) {
@@ -407,9 +633,10 @@ int qb_launch_deltanet(qb_ctx *ctx, const DnArgs &a) {
     QB_REQUIRE(a.conv_out && a.conv_out != a.conv, "deltanet: the new conv state needs a buffer of its own");
     // one request: 32 state columns per CTA (more CTAs, shortest critical path); several: 64 per CTA (the per-CTA
     // work that does not depend on the column count — the head's q/k conv, the barriers — is paid half as often)
-    // prompt ingestion (many rows per sequence): 64 columns per CTA and 8-row blocks
-    const bool wide = a.n_seqs > 2, many = a.rows_per_seq >= 16;
-    if (a.hd == 128) return many ? launch_fused<128, 4, 8, 1>(ctx, a) : wide ? launch_fused<128, 4, 4, 2>(ctx, a) : launch_fused<128, 2, 4, 2>(ctx, a);
-    if (a.hd == 64) return many ? launch_fused<64, 4, 8, 1>(ctx, a) : wide ? launch_fused<64, 4, 4, 2>(ctx, a) : launch_fused<64, 2, 4, 2>(ctx, a);
+    // prompt ingestion (16 rows or more per sequence, only the last state kept): the three-launch form.  Below 16 rows its two more
+    // launches cost what the shorter rows give.
+    const bool wide = a.n_seqs > 2, many = a.rows_per_seq >= 16 && !a.write_all;
+    if (a.hd == 128) return many ? launch_ingest<128>(ctx, a) : wide ? launch_fused<128, 4, 4, 2>(ctx, a) : launch_fused<128, 2, 4, 2>(ctx, a);
+    if (a.hd == 64) return many ? launch_ingest<64>(ctx, a) : wide ? launch_fused<64, 4, 4, 2>(ctx, a) : launch_fused<64, 2, 4, 2>(ctx, a);
     return qb_fail(QB_ERR_UNSUPPORTED, "deltanet: head dim %u unsupported (64/128)", a.hd);
 }

@@ -411,7 +411,8 @@ static int qwen35_batch_alloc(qb_ctx *ctx, qb_batch *b, size_t slots) {
     const uint32_t act_cols = std::max({m->attn_in(), m->dn_in(), 2 * F});
     QB_CUDA(cudaMalloc(&b->mtp_h, (size_t)rows * H * sizeof(float)));
     QB_CUDA(cudaMalloc(&b->embd, (size_t)rows * H * sizeof(float)));
-    QB_CUDA(cudaMalloc(&b->act, (size_t)rows * act_cols * sizeof(float)));
+    b->act_floats = (size_t)rows * act_cols;
+    QB_CUDA(cudaMalloc(&b->act, b->act_floats * sizeof(float)));
     {
         size_t per_row = 0;   // floats of split partials any GEMM of the model can need per row
         auto consider = [&](uint32_t N, uint32_t K, bool always) {
@@ -873,6 +874,7 @@ static int deltanet_block(qb_ctx *ctx, qb_batch *b, const LayerW &L, uint32_t il
     d.conv_out = (b->conv_par ? b->conv[il] : b->conv_alt[il]) + conv_off;
     d.n_slots = K1; d.slot_in = b->sel + rs.seq0; d.write_all = checkpoints ? 1 : 0;
     d.q8 = b->xq_dn.q; d.q_pitch = b->xq_dn.K; d.d = b->xq_dn.d; d.d_ld = qb_act_ld(rows);
+    d.work = b->act; d.work_floats = b->act_floats;          // (free until the feed-forward)
     QB_TRY(qb_launch_deltanet(ctx, d));
     uint32_t S = 1;
     QB_TRY(gemm_parts(ctx, b, L.w_out, b->xq_dn, rows, &S));

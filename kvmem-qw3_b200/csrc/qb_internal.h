@@ -98,9 +98,12 @@ struct qb_ctx {
     size_t scratch_bytes = 0;
     void *scratch2 = nullptr;              // second area for entry points that call another scratch user
     size_t scratch2_bytes = 0;
+    void *scratch3 = nullptr;              // workspace of the DeltaNet ingestion launches when the caller brings none
+    size_t scratch3_bytes = 0;
 };
 int qb_ctx_scratch(qb_ctx *ctx, size_t bytes, void **out);
 int qb_ctx_scratch2(qb_ctx *ctx, size_t bytes, void **out);
+int qb_ctx_scratch3(qb_ctx *ctx, size_t bytes, void **out);
 void qb_trace_mark(qb_ctx *ctx, const char *name);
 uint32_t qb_env_u32(const char *name, uint32_t dflt);
 // Device timeline (qb_debug_timeline_*): while enabled every tensor-core GEMM launch gets a slot of
@@ -317,5 +320,6 @@ struct DnArgs {
     int write_all = 0;
     int8_t *q8 = nullptr; uint32_t q_pitch = 0; float *d = nullptr; uint32_t d_ld = 0;   // quantised gated core
     float *core_out = nullptr;                               // optional fp32 gated core
+    float *work = nullptr; size_t work_floats = 0;           // workspace of the ingestion form; null or too small = the context's
 };
 int qb_launch_deltanet(qb_ctx *ctx, const DnArgs &a);

@@ -1,0 +1,44 @@
+"""The forms that prompts take (many rows at once) against the forms of decode steps: the same bits, at sizes around the edges
+of their blocks."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nk,nv,hd,n_seqs,R", [(16, 48, 128, 1, 16), (2, 4, 128, 2, 33), (4, 4, 128, 1, 41), (2, 4, 64, 3, 31), (1, 3, 64, 1, 17),
+                                               (2, 2, 128, 1, 130)])
+def test_deltanet_prompt_rows_equal_the_same_rows_in_small_parts(qb, ctx, nk, nv, hd, n_seqs, R):
+    """The three-launch ingestion form == the one-kernel form over parts of up to 7 rows: outputs, states and conv windows, bit for bit."""
+    rng = np.random.default_rng(R + hd)
+    n_slots, Cq = 3, (2 * nk + nv) * hd
+    stride = Cq + nv * hd + 2 * nv + 5
+    proj = rng.standard_normal((n_seqs, R, stride)).astype(np.float32)
+    state = (rng.standard_normal((n_seqs, n_slots, nv, hd, hd)) * 0.05).astype(np.float32)
+    conv = rng.standard_normal((n_seqs, n_slots, Cq, 3)).astype(np.float32)
+    cw = ctx.array(rng.uniform(-0.5, 0.5, (Cq, 4)).astype(np.float32))
+    sa = ctx.array((-np.exp(rng.uniform(0, np.log(16), nv))).astype(np.float32))
+    dt = ctx.array(rng.uniform(-4, -1, nv).astype(np.float32))
+    nw = ctx.array(rng.uniform(0.5, 1.5, hd).astype(np.float32))
+    slot0 = rng.integers(0, n_slots, n_seqs).astype(np.int32)
+
+    def run(parts):
+        d_state, d_conv = ctx.array(state), ctx.array(conv)
+        slot, cores, t = slot0, [], 0
+        for n in parts:
+            core = ctx.empty((n_seqs * n, nv * hd), np.float32)
+            qb.binding.check(qb.lib().qb_deltanet_rows(ctx.h, ctx.array(np.ascontiguousarray(proj[:, t:t + n])).ptr, n_seqs, n, stride, cw.ptr, sa.ptr,
+                                                       dt.ptr, nw.ptr, nk, nv, hd, C.c_float(1e-6), d_state.ptr, d_conv.ptr, n_slots,
+                                                       ctx.array(slot).ptr, 0, core.ptr))
+            cores.append(core.download().reshape(n_seqs, n, nv * hd))
+            slot, t = np.zeros(n_seqs, np.int32), t + n
+        return np.concatenate(cores, 1), d_state.download()[:, 0], d_conv.download()[:, 0]
+
+    parts = []
+    while sum(parts) < R:
+        parts.append(min(R - sum(parts), 1 + (3 * len(parts)) % 7))
+    whole, small = run([R]), run(parts)
+    for a, b in zip(whole, small):
+        assert np.array_equal(a, b)
