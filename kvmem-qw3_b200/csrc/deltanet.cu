@@ -11,6 +11,7 @@
 // goes to slot t, so accepting `a` drafts is "slot_in = a" and nothing is copied.  Without checkpoints only
 // the final state is written, to slot 0.
 #include "qb_internal.h"
+#include "tc_common.cuh"
 
 namespace {
 
@@ -362,7 +363,7 @@ int launch_fused(qb_ctx *ctx, const DnArgs &a) {
 // sequential, so for many rows everything else leaves that chain:
 //   dn_prep_kernel   conv + SiLU, L2 norm, gates of all rows at once
 //   dn_scan_kernel   the delta rule; a column of the state is held by 8 lanes (16 of its 128 values each at head size 128): three
-//                    exchange steps instead of five, two of them shared by the columns of a thread; rows arrive by cp.async
+//                    exchange steps instead of five, the first shared by the columns of a thread; rows arrive by cp.async
 //   dn_gate_kernel   head-wide RMSNorm * gain * SiLU(z), quantisation, all rows at once
 // Every sum is formed from the same pairs in the same order as in dn_fused_kernel (a lane adds the partial sums of the four lanes
 // it stands for as the first two exchange steps would), so a row has the same bits in either form.
@@ -371,7 +372,9 @@ constexpr uint32_t DN_PB = 8;                    // rows per block of the two pa
 // q and k are stored so that a lane of the scan reads its values with 16-byte loads: inside every 32 values, index 8j + m is at 4m + j.
 template <int HD>
 __global__ void __launch_bounds__(HD) dn_prep_kernel(DnArgs a, float *__restrict__ qk, float *__restrict__ vc, float *__restrict__ gb) {
-    QB_PDL_ENTER();
+    // No early start of the scan: its CTAs would be placed while this kernel's still fill most SMs, several of them on the SMs that
+    // are free first, and the scan's time is that of its fullest SM (500 us instead of 255 per 512 rows).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float red[DN_PB][HD / 32];
     const uint32_t u = blockIdx.x, rb0 = blockIdx.y * DN_PB, seq = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t R = a.rows_per_seq, nrows = min(DN_PB, R - rb0), ch = u * HD + tid;
@@ -479,14 +482,15 @@ __global__ void __launch_bounds__(32 * NW) dn_scan_kernel(DnArgs a, const float 
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     fetch(0, 0);
-    float s[CPT][NR][4];
+    using namespace qbtc;
+    f32x2 s[CPT][NR][2];                                        // packed arithmetic: half the instructions, each lane rounds as alone
     const float *st_in = a.state + ((size_t)seq * a.n_slots + (uint32_t)a.slot_in[seq]) * ssz + ((size_t)vh * HD + blockIdx.x * COLS + lc) * HD + m;
 #pragma unroll
     for (int c = 0; c < CPT; ++c)
 #pragma unroll
         for (int r = 0; r < NR; ++r)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s[c][r][j] = st_in[(size_t)c * HD + r * 32 + 8 * j];
+            for (int j = 0; j < 2; ++j) s[c][r][j] = pack2(st_in[(size_t)c * HD + r * 32 + 16 * j], st_in[(size_t)c * HD + r * 32 + 16 * j + 8]);
     const float oscale = rsqrtf((float)HD);
     const bool hi4 = (m & 4) != 0, hi2 = (m & 2) != 0;
     // Totals over a column's 8 lanes: the first step (CPT 4: the first two) halves the columns a lane carries.  The lane ends with the
@@ -518,36 +522,43 @@ __global__ void __launch_bounds__(32 * NW) dn_scan_kernel(DnArgs a, const float 
         for (uint32_t t = 0; t < n; ++t) {
             const float *row = buf[bf][t];
             const float g = row[2 * HD + COLS], beta = row[2 * HD + COLS + 1];
-            float4 kr[NR], qr[NR];
+            const f32x2 g2 = pack2(g, g);
+            ulonglong2 kr[NR], qr[NR];
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
-                kr[r] = *reinterpret_cast<const float4 *>(row + HD + r * 32 + 4 * m);
-                qr[r] = *reinterpret_cast<const float4 *>(row + r * 32 + 4 * m);
+                kr[r] = *reinterpret_cast<const ulonglong2 *>(row + HD + r * 32 + 4 * m);
+                qr[r] = *reinterpret_cast<const ulonglong2 *>(row + r * 32 + 4 * m);
             }
+            // sums of the four lanes this one stands for (m, m + 8 | m + 16, m + 24), then the first two exchange steps
+            auto fold = [&](f32x2 lo, f32x2 hi) -> float {
+                float a0, a1, b0, b1;
+                unpack2(lo, a0, a1);
+                unpack2(hi, b0, b1);
+                return (a0 + b0) + (a1 + b1);
+            };
             float part[CPT];
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
-                float p[4] = {0.0f, 0.0f, 0.0f, 0.0f};          // the four lanes this one stands for: m, m + 8, m + 16, m + 24
+                f32x2 lo = pack2(0.0f, 0.0f), hi = lo;
 #pragma unroll
-                for (int r = 0; r < NR; ++r) {
-                    p[0] += s[c][r][0] * kr[r].x; p[1] += s[c][r][1] * kr[r].y; p[2] += s[c][r][2] * kr[r].z; p[3] += s[c][r][3] * kr[r].w;
-                }
-                part[c] = (p[0] + p[2]) + (p[1] + p[3]);
+                for (int r = 0; r < NR; ++r) { lo = fma2(s[c][r][0], kr[r].x, lo); hi = fma2(s[c][r][1], kr[r].y, hi); }
+                part[c] = fold(lo, hi);
             }
             const float kvt = total(part);
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
                 const float kv = __shfl_sync(0xffffffffu, kvt, CPT == 4 ? 4 * (c >> 1) + 2 * (c & 1) : 4 * c, 8);
                 const float delta = (row[2 * HD + lc + c] - g * kv) * beta;
-                float p[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                const f32x2 d2 = pack2(delta, delta);
+                f32x2 lo = pack2(0.0f, 0.0f), hi = lo;
 #pragma unroll
                 for (int r = 0; r < NR; ++r) {
-                    s[c][r][0] = g * s[c][r][0] + kr[r].x * delta; p[0] += s[c][r][0] * qr[r].x;
-                    s[c][r][1] = g * s[c][r][1] + kr[r].y * delta; p[1] += s[c][r][1] * qr[r].y;
-                    s[c][r][2] = g * s[c][r][2] + kr[r].z * delta; p[2] += s[c][r][2] * qr[r].z;
-                    s[c][r][3] = g * s[c][r][3] + kr[r].w * delta; p[3] += s[c][r][3] * qr[r].w;
+                    s[c][r][0] = fma2(g2, s[c][r][0], mul2(kr[r].x, d2));
+                    s[c][r][1] = fma2(g2, s[c][r][1], mul2(kr[r].y, d2));
+                    lo = fma2(s[c][r][0], qr[r].x, lo);
+                    hi = fma2(s[c][r][1], qr[r].y, hi);
                 }
-                part[c] = (p[0] + p[2]) + (p[1] + p[3]);
+                part[c] = fold(lo, hi);
             }
             const float att = total(part);
             if (CPT == 4 ? (m & 1) == 0 : (m & 3) == 0) v_src[(size_t)(t0 + t) * vdim + lc + (CPT == 4 ? m >> 1 : m >> 2)] = att * oscale;
@@ -560,7 +571,12 @@ __global__ void __launch_bounds__(32 * NW) dn_scan_kernel(DnArgs a, const float 
 #pragma unroll
         for (int r = 0; r < NR; ++r)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) st_out[(size_t)c * HD + r * 32 + 8 * j] = s[c][r][j];
+            for (int j = 0; j < 2; ++j) {
+                float x0, x1;
+                unpack2(s[c][r][j], x0, x1);
+                st_out[(size_t)c * HD + r * 32 + 16 * j] = x0;
+                st_out[(size_t)c * HD + r * 32 + 16 * j + 8] = x1;
+            }
 }
 
 template <int HD>
@@ -605,7 +621,9 @@ __global__ void __launch_bounds__(HD) dn_gate_kernel(DnArgs a, const float *__re
 
 template <int HD>
 int launch_ingest(qb_ctx *ctx, const DnArgs &a) {
-    constexpr int CPT = 4, NW = HD == 128 ? 4 : 2;               // 64 (32) columns per CTA
+    // 64 columns per CTA, two per thread.  Measured per 512 rows, all three launches: 2 columns x 8 warps 226 us, 2 x 4 252,
+    // 4 x 4 285, 4 x 2 292, 4 x 1 318.
+    constexpr int CPT = 2, NW = 8;
     const size_t rows = (size_t)a.n_seqs * a.rows_per_seq, nqk = rows * a.nk * 2 * HD, nvc = rows * a.nv * HD, need = nqk + nvc + rows * 2 * a.nv;
     float *work = a.work;
     if (!work || need > a.work_floats) {
