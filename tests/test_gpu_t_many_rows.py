@@ -42,3 +42,28 @@ def test_deltanet_prompt_rows_equal_the_same_rows_in_small_parts(qb, ctx, nk, nv
     whole, small = run([R]), run(parts)
     for a, b in zip(whole, small):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64, 65, 100])
+@pytest.mark.parametrize("N,K,stride", [(64, 32, 32), (130, 100, 101), (9600, 64, 68), (200, 2056, 2056)])
+def test_dense_product_in_32_bits(qb, ctx, M, N, K, stride):
+    """Every tile of the fp32 product (rows and columns around its edges, odd strides) against 64 bits.  An output is four chains of K / 4
+    fused multiply-adds and two additions: at most (K / 4 + 2) roundings of half a unit in the last place of sum |x w|.
+    The same bits whatever the number of rows."""
+    rng = np.random.default_rng(M + N + K)
+    w = (rng.standard_normal((N, K)) * 0.05).astype(np.float32)
+    bits = (w.view(np.uint32) >> 16).astype(np.uint16)
+    w = (bits.astype(np.uint32) << 16).view(np.float32)
+    x = np.full((M, stride), np.nan, np.float32)
+    x[:, :K] = rng.standard_normal((M, K)).astype(np.float32)
+    L, h = qb.lib(), C.c_void_p()
+    qb.binding.check(L.qb_dense_weight(ctx.h, bits.ctypes.data_as(C.c_void_p), N, K, C.byref(h)))
+    xd, y, y1 = ctx.array(x), ctx.empty((M, N), np.float32), ctx.empty((1, N), np.float32)
+    qb.binding.check(L.qb_dense_matmul(ctx.h, h, xd.ptr, M, stride, y.ptr, 1))
+    qb.binding.check(L.qb_dense_matmul(ctx.h, h, xd.ptr, 1, stride, y1.ptr, 1))
+    got, first = y.download(), y1.download()
+    L.qb_dense_weight_free(ctx.h, h)
+    want = x[:, :K].astype(np.float64) @ w.T.astype(np.float64)
+    bound = (K / 4 + 2) * 2.0 ** -24 * (np.abs(x[:, :K]).astype(np.float64) @ np.abs(w.T).astype(np.float64))
+    assert (np.abs(got - want) <= bound).all()
+    assert np.array_equal(got[:1], first)
