@@ -234,14 +234,15 @@ int launch_dense(qb_ctx *ctx, const QbDense &w, const QbActBuf &x, uint32_t M, c
 }
 
 // Activation rows per tile: the smallest that covers M up to 64 rows, else the one with the least estimated time (waves of
-// units over the SMs x tile width / efficiency of the tile).
+// units over the SMs x tile width / efficiency of the tile).  Efficiencies from [1024 rows] x [16384 x 4096] on full waves: 1.04 PFLOP/s with
+// 128 columns (both operands of such an MMA take the shared memory's whole bandwidth), 1.51 with 256.
 uint32_t pick_nt(const QbDense &w, uint32_t M, uint32_t sms) {
     if (M <= 16) return 16;
     if (M <= 32) return 32;
     if (M <= 64) return 64;
     uint32_t best = 64;
     double best_t = 1e300;
-    const struct { uint32_t nt; double eff; } cand[] = {{64, 0.6}, {128, 0.9}, {256, 1.0}};
+    const struct { uint32_t nt; double eff; } cand[] = {{64, 0.4}, {128, 0.7}, {256, 1.0}};
     for (const auto &c : cand) {
         const uint32_t units = (w.rows_pad / 128) * ((M + c.nt - 1) / c.nt);
         const double t = (double)((units + sms - 1) / sms) * c.nt / c.eff;
