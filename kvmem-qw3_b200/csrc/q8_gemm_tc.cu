@@ -25,6 +25,22 @@
 namespace {
 using namespace qbtc;
 
+// 16 lanes x 32 columns: register 4j+i of lane t is row t/4 + 8*(i/2), column 8j + 2*(t%4) + i%2
+__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, int32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait_dep2(int32_t (&r)[16], int32_t (&s)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                   "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(s[0]), "+r"(s[1]), "+r"(s[2]),
+                   "+r"(s[3]), "+r"(s[4]), "+r"(s[5]), "+r"(s[6]), "+r"(s[7]), "+r"(s[8]), "+r"(s[9]), "+r"(s[10]), "+r"(s[11]),
+                   "+r"(s[12]), "+r"(s[13]), "+r"(s[14]), "+r"(s[15]));
+}
+
 // MT = activation rows per tile (MMA N).  NLD = accumulator columns the epilogue reads (<= MT).
 // A pipeline stage holds one weight record (17 KB, one bulk copy, already the swizzled operand image
 // plus its scales), the activation tile (MT x 128 B, tensor-map TMA with the 128-byte swizzle) and
@@ -56,10 +72,9 @@ struct TcCfg {
     static constexpr int NST = NST_FIT > 8 ? 8 : NST_FIT;
     static constexpr int TOTAL = STAGE * NST + BAR_BYTES + EX_BYTES + 1024;   // + slack to align the base to 1024
     static constexpr int CH = NLD < 16 ? NLD : 16;               // columns per tcgen05.ld
-    // Epilogue warps: four for the small tiles (one per TMEM lane quarter); eight from MT = 32 and sixteen at
-    // MT = 128 (two / four per quarter, each taking a slice of the activation columns): the drain + rescale of a
-    // large tile is bound by instruction issue and dependent latencies, which more warps per scheduler hide.
-    static constexpr int EPI_WARPS = MT >= 64 ? 16 : MT >= 32 ? 8 : 4;
+    // Epilogue warps: four for the small tiles (one per TMEM lane quarter), eight or sixteen for the larger ones (two / four per
+    // quarter, each taking a slice of the activation columns).
+    static constexpr int EPI_WARPS = MT == 64 ? 16 : MT >= 32 ? 8 : 4;
     static constexpr int THREADS = 64 + 32 * EPI_WARPS;
     static constexpr int NC = NLD / (EPI_WARPS / 4);             // accumulator columns per epilogue thread
 };
@@ -251,8 +266,8 @@ gemm_tc_kernel(const uint8_t *__restrict__ rec, const __grid_constant__ CUtensor
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_tempty + 8 * slot);
                 }
-            } else {
-                // Large activation tiles: this warp drains columns [c_base, c_base + NC) of its lane quarter.  The
+            } else if constexpr (MT < 128) {
+                // Middling activation tiles: this warp drains columns [c_base, c_base + NC) of its lane quarter.  The
                 // TMEM loads are software-pipelined: the next 16 columns are in flight while the current 16 are
                 // rescaled.
                 constexpr int NC = C::NC, NCH = NC / 16;                // 16-column chunks per 32-block
@@ -303,6 +318,84 @@ gemm_tc_kernel(const uint8_t *__restrict__ rec, const __grid_constant__ CUtensor
                 }
 #pragma unroll
                 for (int i = 0; i < NC / 2; ++i) unpack2(acc2[i], acc[2 * i], acc[2 * i + 1]);
+            } else {
+                // The 128-row tile.  The 16x256b loads give a thread four rows x every fourth pair of columns, so it reads NC / 4 activation scales
+                // per block and not NC: a scale that every lane reads costs its full width in shared-memory wavefronts (13 M of them in a
+                // 17408 x 5120 x 128 product with the 32x32b loads, which give one row x all columns).  Eight warps of 64 columns, 34816 x 5120: 142 ->
+                // 136 us with 128 rows, 522 -> 500 with 512 (16 warps of 32: 154 and 565; at 64 rows and below no gain: 80 against 78).  The
+                // two loads of a half are waited for at once: with the next half's in flight behind them 167 and 620.
+                constexpr int NC = C::NC;
+                const uint32_t r0 = quarter * 32 + (lane >> 2), cw = ((warp - 2) >> 2) * NC, c0 = cw + 2 * (lane & 3);
+                f32x2 a2[NC / 8][4];                                    // [column pair][row]
+#pragma unroll
+                for (int i = 0; i < NC / 8; ++i)
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) a2[i][p] = pack2(0.0f, 0.0f);
+                for (uint32_t it = 0; it < n_it && ok; ++it, ++git) {
+                    const uint32_t st = git % NST;                      // (landed: the slot barrier implies it)
+                    const uint8_t *stage = smem + (size_t)st * C::STAGE;
+                    const __half *wd = reinterpret_cast<const __half *>(stage + QB_REC_Q_BYTES) + r0;
+                    const float *xd = reinterpret_cast<const float *>(stage + C::XD_OFF) + c0;
+                    for (int sp = 0; sp < C::SPS; ++sp, ++j) {
+                        const uint32_t slot = j % NSLOT, sph = (j / NSLOT) & 1;
+                        if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * slot, sph, abort_flag))) { ok = false; break; }
+                        tc_fence_after();
+                        const uint32_t t = tmem_base + ((quarter * 32u) << 16) + slot * (C::KPS * MT) + cw;
+#pragma unroll
+                        for (int kl = 0; kl < C::KPS; ++kl) {
+                            const int kb = sp * C::KPS + kl;
+                            f32x2 dw[4];
+#pragma unroll
+                            for (int p = 0; p < 4; ++p) { const float f = __half2float(wd[kb * 128 + 8 * p]); dw[p] = pack2(f, f); }
+#pragma unroll
+                            for (int h = 0; h < NC / 32; ++h) {
+                                int32_t va[16], vb[16];
+                                tmem_ld_16x256b_x4(t + kl * MT + h * 32, va);
+                                tmem_ld_16x256b_x4(t + (16u << 16) + kl * MT + h * 32, vb);
+                                f32x2 x[4];
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) x[q] = *reinterpret_cast<const f32x2 *>(xd + kb * MT + h * 32 + 8 * q);
+                                tmem_wait_dep2(va, vb);
+                                if (h == NC / 32 - 1 && kl == C::KPS - 1) {       // the whole slot is in registers
+                                    tc_fence_before();
+                                    __syncwarp();
+                                    if (lane == 0) mbar_arrive(bar_tempty + 8 * slot);
+                                }
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) {
+                                    f32x2 (&a)[4] = a2[h * 4 + q];
+                                    a[0] = fma2(mul2(dw[0], x[q]), pack2((float)va[4 * q], (float)va[4 * q + 1]), a[0]);
+                                    a[1] = fma2(mul2(dw[1], x[q]), pack2((float)va[4 * q + 2], (float)va[4 * q + 3]), a[1]);
+                                    a[2] = fma2(mul2(dw[2], x[q]), pack2((float)vb[4 * q], (float)vb[4 * q + 1]), a[2]);
+                                    a[3] = fma2(mul2(dw[3], x[q]), pack2((float)vb[4 * q + 2], (float)vb[4 * q + 3]), a[3]);
+                                }
+                            }
+                        }
+                    }
+                    if (ok) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_empty + 8 * st);
+                    }
+                }
+                if (ok) {
+#pragma unroll
+                    for (int i = 0; i < NC / 4; ++i) {
+                        const uint32_t m = m0 + c0 + 8 * (i / 2) + (i & 1);
+                        if (m >= M) continue;
+#pragma unroll
+                        for (int p = 0; p < 4; ++p) {
+                            const uint32_t row = tile * 128 + r0 + 8 * p;
+                            if (row >= N) continue;
+                            float lo, hi;
+                            unpack2(a2[i / 2][p], lo, hi);
+                            const float val = (i & 1) ? hi : lo;
+                            const size_t o = ((size_t)seg * M + m) * N + row;
+                            if (push.n == 0) part[o] = val;
+                            else for (uint32_t d = 0; d < push.n; ++d) push.dst[d][o] = val;
+                        }
+                    }
+                }
+                continue;
             }
             if constexpr (MT == 16) {
                 if (swz.q != nullptr) {
