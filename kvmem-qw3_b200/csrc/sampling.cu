@@ -22,7 +22,7 @@ namespace {
 
 constexpr int ST = 1024;                      // threads per CTA
 constexpr int CL = 8;                         // CTAs per row (one cluster)
-constexpr int EPT = 20;                       // elements per thread at most: rows up to CL * ST * EPT = 163840 logits
+constexpr int EPT_MAX = 20;                   // elements per thread at most: rows up to CL * ST * EPT_MAX = 163840 logits
 constexpr int NB = 4;                         // histogram bins per pass (two key bits)
 
 struct SampleParams {
@@ -154,6 +154,7 @@ __device__ void block_exscan(Comm &c, double v, long long n, double &ex_v, long 
 // One cluster per row.  draft == nullptr or the row's draft < 0: no draft (bonus / plain sampling row).
 // K1 = 0: one draft entry per row; K1 > 0: rows are [sequence][K1] and drafts [sequence][K1 - 1], the last row of a
 // sequence has none.
+template <int EPT>
 __global__ void __launch_bounds__(ST)
 sample_rows_kernel(const float *__restrict__ logits, uint32_t V, uint32_t stride, const int32_t *__restrict__ draft,
                    const double *__restrict__ u_acc, const double *__restrict__ u_res, SampleParams p, int32_t *token,
@@ -416,7 +417,7 @@ int qb_launch_sample_rows(qb_ctx *ctx, const float *logits, uint32_t rows, uint3
     p.inv_t = 1.0f / temp; p.top_p = top_p; p.min_p = min_p; p.top_k = top_k;
     p.presence = presence; p.repetition = repetition; p.seen = seen; p.seen_words = seen_words;
     p.chain_limit = chain_limit; p.eos = eos;
-    QB_REQUIRE(V <= (uint32_t)(CL * ST * EPT), "sampling: rows of %u logits exceed the kernel's %d", V, CL * ST * EPT);
+    QB_REQUIRE(V <= (uint32_t)(CL * ST * EPT_MAX), "sampling: rows of %u logits exceed the kernel's %d", V, CL * ST * EPT_MAX);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * CL);
     cfg.blockDim = dim3(ST);
@@ -430,7 +431,9 @@ int qb_launch_sample_rows(qb_ctx *ctx, const float *logits, uint32_t rows, uint3
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    QB_CUDA(cudaLaunchKernelEx(&cfg, sample_rows_kernel, logits, V, stride, draft, u_acc, u_res, p, token, accepted, p_draft, pval,
+    // the loops over a thread's elements are unrolled: vocabularies up to 32768 take the form with 4 of them
+    const auto kernel = V <= (uint32_t)(CL * ST * 4) ? sample_rows_kernel<4> : sample_rows_kernel<EPT_MAX>;
+    QB_CUDA(cudaLaunchKernelEx(&cfg, kernel, logits, V, stride, draft, u_acc, u_res, p, token, accepted, p_draft, pval,
                                pidx, nblk, K1));
     QB_LAUNCHED(ctx, "sample_rows_kernel");
     return QB_OK;
