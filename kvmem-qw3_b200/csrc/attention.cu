@@ -487,9 +487,85 @@ __global__ void __launch_bounds__(1024) attn_merge_kernel(AttnArgs a, const int3
     }
 }
 
+// The same merge for up to 32 splits: four consecutive values a thread, hd / 4 threads a (row, head), weights recomputed by each thread instead
+// of passed through shared memory -- no barrier and no idle group; the same sums in the same order.  A prompt pass of 2048 rows x 24 heads
+// of 256 with up to 9 splits: 500 -> 188 us; 128 rows 14.2 -> 7.7; bound by reading the partials.  Under 64 rows the chain over the splits is
+// the longer one (4 rows, 17 splits: 8.8 against 5.7).
+constexpr uint32_t MERGE4_SPLITS = 32, MERGE4_THREADS = 256, MERGE4_MIN_ROWS = 64;
+__global__ void __launch_bounds__(MERGE4_THREADS) attn_merge4_kernel(AttnArgs a, const int32_t *__restrict__ seq_pos, uint32_t R, uint32_t max_splits,
+                                                                     float *out, int8_t *q8, uint32_t q_pitch, float *dsc, uint32_t d_ld) {
+    QB_PDL_ENTER();
+    const uint32_t hd = a.hd, per = hd / 4, unit = blockIdx.x * (MERGE4_THREADS / per) + threadIdx.x / per, i = threadIdx.x % per * 4;
+    const bool in = unit < a.rows * a.n_heads;
+    const uint32_t row = in ? unit / a.n_heads : 0, head = in ? unit % a.n_heads : 0;
+    const int pos = seq_pos[row / R] + (int)(row % R);
+    const uint32_t nsplit = ((uint32_t)pos + a.split_keys) / a.split_keys;
+    const size_t p0 = ((size_t)row * a.n_heads + head) * max_splits;
+    const float2 *ml = reinterpret_cast<const float2 *>(a.part_ml) + p0;
+    float mx = -INFINITY;
+#pragma unroll 8
+    for (uint32_t s = 0; s < nsplit; ++s) mx = fmaxf(mx, ml[s].x);
+    float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+    float den = 0.0f;
+    for (uint32_t sb = 0; sb < nsplit; sb += MERGE_BLOCK) {
+        const float *acc = a.part_acc + (p0 + sb) * hd + i;
+        float4 n4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        float d1 = 0.0f;
+#pragma unroll
+        for (uint32_t h = 0; h < MERGE_BLOCK; h += 8) {
+            float4 va[8];
+            float2 w[8];
+#pragma unroll
+            for (uint32_t u = 0; u < 8; ++u)
+                if (sb + h + u < nsplit) { va[u] = *reinterpret_cast<const float4 *>(acc + (size_t)(h + u) * hd); w[u] = ml[sb + h + u]; }
+#pragma unroll
+            for (uint32_t u = 0; u < 8; ++u)
+                if (sb + h + u < nsplit) {
+                    const float e = expf(w[u].x - mx);
+                    n4.x = fmaf(va[u].x, e, n4.x); n4.y = fmaf(va[u].y, e, n4.y); n4.z = fmaf(va[u].z, e, n4.z); n4.w = fmaf(va[u].w, e, n4.w);
+                    d1 = fmaf(w[u].y, e, d1);
+                }
+        }
+        num.x += n4.x; num.y += n4.y; num.z += n4.z; num.w += n4.w;
+        den += d1;
+    }
+    float4 o = make_float4(__fdiv_rn(num.x, den), __fdiv_rn(num.y, den), __fdiv_rn(num.z, den), __fdiv_rn(num.w, den));
+    if (!a.no_gate) {
+        const float *gp = a.qkv + (size_t)row * a.row_stride + (size_t)head * 2 * hd + hd + i;
+        float4 g = *reinterpret_cast<const float4 *>(gp);
+        for (uint32_t s = 1; s < a.in_S; ++s) {
+            const float4 p = *reinterpret_cast<const float4 *>(gp + s * a.in_pstride);
+            g.x += p.x; g.y += p.y; g.z += p.z; g.w += p.w;
+        }
+        o.x *= __fdiv_rn(1.0f, 1.0f + expf(-g.x)); o.y *= __fdiv_rn(1.0f, 1.0f + expf(-g.y));
+        o.z *= __fdiv_rn(1.0f, 1.0f + expf(-g.z)); o.w *= __fdiv_rn(1.0f, 1.0f + expf(-g.w));
+    }
+    float amax = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(o.w)));
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    if (!in) return;
+    const uint32_t col = head * hd + i;
+    if (out) *reinterpret_cast<float4 *>(out + (size_t)row * a.n_heads * hd + col) = o;
+    if (q8) {
+        const float d_inv = (amax == 0.0f) ? 0.0f : __fdiv_rn(127.0f, amax);
+        auto quant = [&](float x) -> int8_t { return (int8_t)((amax == 0.0f) ? 0 : __float2int_rn(__fmul_rn(x, d_inv))); };
+        *reinterpret_cast<char4 *>(q8 + (size_t)row * q_pitch + col) = make_char4(quant(o.x), quant(o.y), quant(o.z), quant(o.w));
+        if ((i & 31) == 0) dsc[(size_t)(col / 32) * d_ld + row] = (amax == 0.0f) ? 0.0f : __fdiv_rn(1.0f, d_inv);
+    }
+}
+
 // One place for the merge launch: NG thread groups by the host's bound of the split count (the result does not depend on NG).
 static int launch_merge(qb_ctx *ctx, const AttnArgs &aa, const int32_t *seq_pos, uint32_t R, uint32_t ms, float *out, int8_t *q8,
                         uint32_t q_pitch, float *d, uint32_t d_ld) {
+    const bool vec = ((uintptr_t)aa.qkv & 15) == 0 && aa.row_stride % 4 == 0 && aa.in_pstride % 4 == 0 && ((uintptr_t)aa.part_acc & 15) == 0 && ((uintptr_t)aa.part_ml & 7) == 0 &&
+                     ((uintptr_t)out & 15) == 0 && ((uintptr_t)q8 & 3) == 0 && q_pitch % 4 == 0;
+    if (vec && aa.rows >= MERGE4_MIN_ROWS && ms <= MERGE4_SPLITS && aa.hd % 32 == 0 && aa.hd <= 4 * MERGE4_THREADS && MERGE4_THREADS % (aa.hd / 4) == 0) {
+        const uint32_t per_cta = MERGE4_THREADS / (aa.hd / 4);
+        QB_CUDA(qb_launch_pdl(ctx->stream, attn_merge4_kernel, dim3((aa.rows * aa.n_heads + per_cta - 1) / per_cta), dim3(MERGE4_THREADS), (size_t)0, aa, seq_pos, R, ms, out, q8,
+                              q_pitch, d, d_ld));
+        QB_LAUNCHED(ctx, "attn_merge_kernel");
+        return QB_OK;
+    }
     const uint32_t nb_max = (ms + MERGE_BLOCK - 1) / MERGE_BLOCK;
     const uint32_t ng = std::max(1u, std::min(std::min(nb_max, 1024u / aa.hd), 8u));
     const size_t smem = (size_t)nb_max * (aa.hd + 1) * sizeof(float);
