@@ -245,11 +245,46 @@ __global__ void swiglu_quant_kernel(const float *__restrict__ gu, uint32_t gu_st
     quant_block_store(qb_swiglu(g, u), lane, q + (size_t)m * q_pitch + b * 32, d + (size_t)b * d_ld + m);
 }
 
+// The same with 16-byte loads, four hidden indices a thread and eight threads a 32-block (bound by the bytes of gate and up: 2048 rows
+// of 2 x 17408, one K segment, 240 -> 79 us).  Needs every 4-element piece aligned; gate and up groups are whole pieces.
+__global__ void __launch_bounds__(256) swiglu_quant4_kernel(const float *__restrict__ gu, uint32_t gu_stride, uint32_t F, int8_t *q,
+                                                            uint32_t q_pitch, float *d, uint32_t d_ld, uint32_t S, size_t pstride, uint32_t ileave) {
+    QB_PDL_ENTER();
+    const uint32_t c = (blockIdx.x * 256 + threadIdx.x) * 4, m = blockIdx.y, lane = threadIdx.x & 31;
+    const bool in = c < F;                                               // whole blocks: F is a multiple of 32
+    const uint32_t gi = ileave ? (c / ileave) * 2 * ileave + c % ileave : c, ui = ileave ? gi + ileave : F + c;
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f), u = g;
+    if (in) {
+        const float *row = gu + (size_t)m * gu_stride;
+        g = *reinterpret_cast<const float4 *>(row + gi);
+        u = *reinterpret_cast<const float4 *>(row + ui);
+        for (uint32_t s = 1; s < S; ++s) {
+            const float4 pg = *reinterpret_cast<const float4 *>(row + s * pstride + gi), pu = *reinterpret_cast<const float4 *>(row + s * pstride + ui);
+            g.x += pg.x; g.y += pg.y; g.z += pg.z; g.w += pg.w;
+            u.x += pu.x; u.y += pu.y; u.z += pu.z; u.w += pu.w;
+        }
+    }
+    const float4 v = make_float4(qb_swiglu(g.x, u.x), qb_swiglu(g.y, u.y), qb_swiglu(g.z, u.z), qb_swiglu(g.w, u.w));
+    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (!in) return;
+    const float d_inv = (amax == 0.0f) ? 0.0f : __fdiv_rn(127.0f, amax);     // as quant_block_store
+    auto quant = [&](float x) -> int8_t { return (int8_t)((amax == 0.0f) ? 0 : __float2int_rn(__fmul_rn(x, d_inv))); };
+    *reinterpret_cast<char4 *>(q + (size_t)m * q_pitch + c) = make_char4(quant(v.x), quant(v.y), quant(v.z), quant(v.w));
+    if ((lane & 7) == 0) d[(size_t)(c >> 5) * d_ld + m] = (amax == 0.0f) ? 0.0f : __fdiv_rn(1.0f, d_inv);
+}
+
 int qb_launch_swiglu_quant(qb_ctx *ctx, const float *gu, uint32_t gu_stride, uint32_t M, uint32_t F, int8_t *q,
                            uint32_t q_pitch, float *d, uint32_t d_ld, uint32_t S, size_t pstride, uint32_t ileave) {
-    dim3 grid((F / 32 + 7) / 8, M);
-    QB_CUDA(qb_launch_pdl(ctx->stream, swiglu_quant_kernel, dim3(grid), dim3(256), (size_t)(0), gu, gu_stride, F, q, q_pitch, d, d_ld, S, pstride,
-                          ileave));
+    const bool vec = ((uintptr_t)gu & 15) == 0 && gu_stride % 4 == 0 && pstride % 4 == 0 && F % 32 == 0 && ileave % 4 == 0 && ((uintptr_t)q & 3) == 0 &&
+                     q_pitch % 4 == 0;
+    if (vec)
+        QB_CUDA(qb_launch_pdl(ctx->stream, swiglu_quant4_kernel, dim3((F + 1023) / 1024, M), dim3(256), (size_t)(0), gu, gu_stride, F, q, q_pitch, d, d_ld, S,
+                              pstride, ileave));
+    else
+        QB_CUDA(qb_launch_pdl(ctx->stream, swiglu_quant_kernel, dim3((F / 32 + 7) / 8, M), dim3(256), (size_t)(0), gu, gu_stride, F, q, q_pitch, d, d_ld, S,
+                              pstride, ileave));
     QB_LAUNCHED(ctx, "swiglu_quant_kernel");
     return QB_OK;
 }
