@@ -180,6 +180,51 @@ __global__ void __launch_bounds__(NQ_THREADS) norm_quant_kernel(NormQuantArgs a,
     if (!a.w) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // complete the opening arrive
 }
 
+// From 256 rows on (up to 8192 elements each): one CTA per row, no cluster -- with rows enough for every SM the eight-fold split only
+// multiplies barriers (2048 rows of 5120 with six or seven partial sums: 140 -> 104 us; at 128 rows it is the slower one, 11.0 against 6.6).  A thread stands for the thread of the same index in four of the eight
+// CTAs of norm_quant_kernel, so every sum is formed from the same parts in the same order.
+constexpr uint32_t NQR_THREADS = 512, NQR_MIN_ROWS = 256;
+__global__ void __launch_bounds__(NQR_THREADS, 2) norm_quant_rows_kernel(NormQuantArgs a, uint32_t vec) {
+    QB_PDL_ENTER();
+    __shared__ float red[NQ_CLUSTER][NQ_THREADS / 32];
+    constexpr int NV = NQ_CLUSTER * NQ_THREADS / NQR_THREADS;            // virtual CTAs per thread: ranks half, half + 2, ...
+    const uint32_t m = blockIdx.x, half = threadIdx.x / NQ_THREADS, tid = threadIdx.x % NQ_THREADS, lane = tid & 31, warp = tid >> 5, sub = tid & 7;
+    const uint32_t nblk = a.n / 32, per = (nblk + NQ_CLUSTER - 1) / NQ_CLUSTER;
+    const NqRow r = nq_row(a, m, vec);
+    float4 v[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const uint32_t rank = half + 2 * k, b0 = rank * per, b1 = min(nblk, b0 + per), b = b0 + (tid >> 3);
+        float ss = 0.0f;
+        float4 g;
+        v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (b < b1) nq_load(a, r, b * 32 + sub * 4, v[k], g, ss);
+        if (a.w) {
+            ss = warp_sum(ss);
+            if (lane == 0) red[rank][warp] = ss;
+        }
+    }
+    float scale = 1.0f;
+    if (a.w) {
+        __syncthreads();
+        float tot = 0.0f;
+#pragma unroll
+        for (int c = 0; c < (int)NQ_CLUSTER; ++c) {
+            float part = 0.0f;
+#pragma unroll
+            for (int i = 0; i < (int)NQ_THREADS / 32; ++i) part += red[c][i];
+            tot += part;
+        }
+        scale = rsqrtf(tot / (float)a.n + a.eps);
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const uint32_t b0 = (half + 2 * k) * per, b1 = min(nblk, b0 + per), b = b0 + (tid >> 3), i = b * 32 + sub * 4;
+        if (b >= b1) continue;          // whole 8-thread groups leave together; the shuffles stay inside a group
+        nq_finish(a, r, m, b, i, lane, v[k], a.w ? ld4(a.w + i, true) : make_float4(1.f, 1.f, 1.f, 1.f), scale);
+    }
+}
+
 template <int P>
 static cudaError_t launch_norm_quant(cudaStream_t stream, const NormQuantArgs &a, uint32_t vec) {
     cudaLaunchConfig_t cfg = {};
@@ -206,7 +251,8 @@ int qb_launch_norm_quant(qb_ctx *ctx, const NormQuantArgs &a) {
                a.q_pitch % 4 == 0 && a.q_col_off % 4 == 0, "norm_quant: gain / output buffers must be 16-byte aligned");
     auto al = [](const void *p, size_t stride) { return ((uintptr_t)p & 15) == 0 && stride % 4 == 0; };
     const uint32_t vec = (al(a.x, a.x_stride) ? 1u : 0u) | (al(a.parts, a.part_ld) ? 2u : 0u) | (al(a.h_out, a.h_stride) ? 4u : 0u);
-    if (per <= 32) QB_CUDA(launch_norm_quant<1>(ctx->stream, a, vec));
+    if (per <= 32 && a.M >= NQR_MIN_ROWS) QB_CUDA(qb_launch_pdl(ctx->stream, norm_quant_rows_kernel, dim3(a.M), dim3(NQR_THREADS), (size_t)0, a, vec));
+    else if (per <= 32) QB_CUDA(launch_norm_quant<1>(ctx->stream, a, vec));
     else if (per <= 64) QB_CUDA(launch_norm_quant<2>(ctx->stream, a, vec));
     else QB_CUDA(launch_norm_quant<4>(ctx->stream, a, vec));
     QB_LAUNCHED(ctx, "norm_quant_kernel");

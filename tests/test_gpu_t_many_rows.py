@@ -67,3 +67,79 @@ def test_dense_product_in_32_bits(qb, ctx, M, N, K, stride):
     bound = (K / 4 + 2) * 2.0 ** -24 * (np.abs(x[:, :K]).astype(np.float64) @ np.abs(w.T).astype(np.float64))
     assert (np.abs(got - want) <= bound).all()
     assert np.array_equal(got[:1], first)
+
+
+@pytest.mark.parametrize("n", [32, 96, 1024, 2080, 5120, 8192])
+@pytest.mark.parametrize("M", [255, 256, 301])
+def test_norm_and_quantiser_of_many_rows_equal_few_rows(qb, ctx, M, n):
+    """RMS norm and activation quantiser: a row has the same bits whether its launch takes the one-CTA or the cluster form."""
+    rng = np.random.default_rng(n + M)
+    x = rng.standard_normal((M, n)).astype(np.float32)
+    x[3] = 0.0
+    w = ctx.array(rng.uniform(0.5, 1.5, n).astype(np.float32))
+    L = qb.lib()
+
+    def norm(rows):
+        out = ctx.empty(rows.shape, np.float32)
+        qb.binding.check(L.qb_rms_norm(ctx.h, ctx.array(rows).ptr, w.ptr, len(rows), n, n, C.c_float(1e-6), out.ptr))
+        return out.download()
+
+    def quant(rows):
+        ld = (len(rows) + 3) // 4 * 4
+        q, d = ctx.empty((len(rows), n), np.int8), ctx.empty((n // 32, ld), np.float32)
+        qb.binding.check(L.qb_quantize_act(ctx.h, ctx.array(rows).ptr, len(rows), n, n, q.ptr, d.ptr))
+        return q.download(), d.download()[:, :len(rows)]
+
+    cut = 77
+    whole = norm(x)
+    assert np.array_equal(whole, np.concatenate([norm(x[i:i + cut]) for i in range(0, M, cut)]))
+    q, d = quant(x)
+    parts = [quant(x[i:i + cut]) for i in range(0, M, cut)]
+    assert np.array_equal(q, np.concatenate([p[0] for p in parts])) and np.array_equal(d, np.concatenate([p[1] for p in parts], 1))
+
+
+@pytest.mark.parametrize("M", [16, 17, 65, 130])
+def test_feed_forward_input_of_many_rows_equals_one_launch_form(qb, orc, ctx, M):
+    """silu(gate) * up quantised by the vectorised kernel (any rows) == the GEMM's own epilogue (up to 16 rows at a time)."""
+    rng = np.random.default_rng(M)
+    F, K = 18944, 1152                                       # one K segment (296 row tiles), K > 1024: the one-launch form applies
+    w = qb.Weight.synth(ctx, 11, 5, 2 * F, K, 0.02)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    L = qb.lib()
+
+    def run(rows, mode):
+        ld = (len(rows) + 3) // 4 * 4
+        q, d = ctx.empty((len(rows), F), np.int8), ctx.empty((F // 32, ld), np.float32)
+        qb.binding.check(L.qb_q8_0_matmul_silu_mul_q8(ctx.h, w.h, ctx.array(rows).ptr, len(rows), K, q.ptr, d.ptr, mode))
+        return q.download(), d.download()[:, :len(rows)]
+
+    q, d = run(x, 1)
+    parts = [run(x[i:i + 16], 2) for i in range(0, M, 16)]
+    assert np.array_equal(q, np.concatenate([p[0] for p in parts])) and np.array_equal(d, np.concatenate([p[1] for p in parts], 1))
+    w.free()
+
+
+@pytest.mark.parametrize("rows,pos,heads,kv,hd", [(64, 0, 6, 2, 256), (65, 300, 24, 4, 256), (80, 2500, 4, 2, 256)])
+def test_merge_of_many_rows_equals_few_rows(qb, ctx, monkeypatch, rows, pos, heads, kv, hd):
+    """Attention over the paged cache with its gate: a row's output has the same bits in a launch of 64 rows and more (splits merged
+    without shared memory) and in parts of 16.  Parts of up to 8 rows would take the tcgen05 splits, whose last bits differ: off."""
+    monkeypatch.setenv("QW3B200_ATTN_TC", "0")
+    rng = np.random.default_rng(rows + pos)
+    page, n_pages = 16, (pos + rows + 15) // 16
+    stride = 2 * heads * hd + 2 * kv * hd
+    qkv = rng.standard_normal((rows, stride)).astype(np.float32)
+    k = ctx.array((rng.standard_normal((n_pages * page, kv, hd)) * 0.3).astype(np.float16))
+    v = ctx.array(rng.standard_normal((n_pages * page, kv, hd)).astype(np.float16))
+    table = ctx.array(np.arange(n_pages, dtype=np.int32)[None])
+
+    def run(lo, hi):
+        out = ctx.empty((hi - lo, heads * hd), np.float32)
+        qb.binding.check(qb.lib().qb_attention_paged_gated(ctx.h, ctx.array(qkv[lo:hi]).ptr, hi - lo, stride, heads, kv, hd,
+                                                           ctx.array(np.array([pos + lo], np.int32)).ptr, 1, table.ptr, n_pages, page, k.ptr, v.ptr,
+                                                           pos + rows, out.ptr))
+        return out.download()
+
+    whole = run(0, rows)
+    parts = np.concatenate([run(lo, min(lo + 16, rows)) for lo in range(0, rows, 16)])
+    assert np.isfinite(whole).all()
+    np.testing.assert_array_equal(whole, parts)
