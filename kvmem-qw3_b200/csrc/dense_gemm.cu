@@ -79,7 +79,7 @@ dense_gemm_kernel(const uint8_t *__restrict__ rec, const __grid_constant__ CUten
     };
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             struct Cursor { uint32_t u, it, n_it, tile, m0, c_begin; bool valid; };
             auto start = [&](uint32_t u) {
                 Cursor c; c.u = u; c.it = 0; c.valid = u < units; c.n_it = 0; c.tile = c.m0 = c.c_begin = 0;
@@ -109,7 +109,7 @@ dense_gemm_kernel(const uint8_t *__restrict__ rec, const __grid_constant__ CUten
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // instruction descriptor: D fp32, A = B = bf16, both K-major, N = NT, M = 128
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) | ((128u >> 4) << 24);
             uint32_t git = 0, j = 0;

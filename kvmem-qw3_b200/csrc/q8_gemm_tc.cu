@@ -141,7 +141,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ rec, const __grid_constant__ CUtensor
     };
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // Stage cursor over this CTA's units.  The launch is programmatically serialised behind the kernel
             // that produces the activations: the weight records of the first NST stages (which depend on nothing)
             // are requested at once, then the CTA waits for the preceding grid and only then requests activations.
@@ -181,7 +181,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ rec, const __grid_constant__ CUtensor
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // instruction descriptor: D = s32, A = B = signed 8-bit, both K-major, N = MT, M = 128
             constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MT >> 3) << 17) | ((128u >> 4) << 24);
             uint32_t git = 0, j = 0;
