@@ -359,7 +359,7 @@ int launch_fused(qb_ctx *ctx, const DnArgs &a) {
 
 // ---- prompt ingestion: three launches per layer ---------------------------------------------------------------
 // One CTA of dn_fused_kernel spends most of a row waiting: two five-step exchanges over 32 lanes, the barriers of the conv and
-// norm phases, one CTA per SM (1.16 us per row, 595 us per 512 rows and layer at 48 heads of 128).  Only the delta rule is
+// norm phases, one CTA per SM (595 us per 512 rows and layer at 48 heads of 128; these three 220, the scan 175).  Only the delta rule is
 // sequential, so for many rows everything else leaves that chain:
 //   dn_prep_kernel   conv + SiLU, L2 norm, gates of all rows at once
 //   dn_scan_kernel   the delta rule; a column of the state is held by 8 lanes (16 of its 128 values each at head size 128): three
