@@ -463,11 +463,13 @@ static int batch_create(qb_ctx *ctx, qb_model *m, uint32_t n_seqs, uint32_t max_
     b->pages_per_seq = (max_ctx + draft_k + 1 + page_size - 1) / page_size;
     // Rows of an ingestion pass: the family's, doubled up to 2048 while the context has use for them (fewer half-empty waves of
     // GEMM tiles and fewer launches: 2048 tokens in passes of 512 / 1024 / 2048: 391 / 378 / 372 ms on the 27B shape; of 1024 / 2048:
-    // 10.1 / 9.4 and 13.0 / 11.7 ms on the layered models) and rows x context stays at what 512 rows take at 32768 (the
-    // attention's split partials grow with that product).  A shard keeps its size: its peers' receive areas are made for it.
+    // 10.1 / 9.4 and 13.0 / 11.7 ms on the layered models) and, for the hybrid, rows x context stays at what 512 rows take at 32768 (the
+    // attention's split partials grow with that product).  A layered model's rows depend on where its passes end (a pass of up to 64 rows
+    // takes split products, one of up to 16 the absorbed attention), so its size follows nothing but whether one pass holds the whole
+    // context: the same prompt gives the same bits at every max_ctx.  A shard keeps its size: its peers' receive areas are made for it.
     uint32_t chunk = m->arch->chunk;
     if (m->tp_world == 1)
-        while (chunk < 2048 && chunk < max_ctx && (size_t)2 * chunk * max_ctx <= (size_t)512 * 32768) chunk *= 2;
+        while (chunk < 2048 && chunk < max_ctx && (m->layered || (size_t)2 * chunk * max_ctx <= (size_t)512 * 32768)) chunk *= 2;
     b->chunk = std::max(1u, qb_env_u32("QW3B200_PREFILL_CHUNK", chunk));
     b->logit_rows = n_seqs * (draft_k + 1);
     b->rows_cap = std::max(b->chunk, b->logit_rows);

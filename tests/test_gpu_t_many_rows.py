@@ -143,3 +143,28 @@ def test_merge_of_many_rows_equals_few_rows(qb, ctx, monkeypatch, rows, pos, hea
     parts = np.concatenate([run(lo, min(lo + 16, rows)) for lo in range(0, rows, 16)])
     assert np.isfinite(whole).all()
     np.testing.assert_array_equal(whole, parts)
+
+
+def prompt_logits(qb, model, toks, max_ctx):
+    b = qb.Batch(model, 1, max_ctx, 0)
+    b.prefill(0, toks)
+    out = b.last_logits(1).copy()
+    rows = b.max_rows
+    b.close()
+    return out, rows
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("family", ["kezilix", "figonex"])
+def test_layered_prompt_does_not_depend_on_the_capacity(qb, ctx, family, dtype):
+    """The end of a layered prompt takes other forms where its pass is short, so passes must end at the same tokens in every batch:
+    the same logits, bit for bit, whatever max_ctx (1030: six tokens past 1024; 2060: the second pass of every batch)."""
+    make = qb.configs.kezilix_bench if family == "kezilix" else qb.configs.figonex_bench
+    m = qb.Model.layered_synth(ctx, make(512, 1024, 4, vocab=512), 3, dtype)
+    for n in (1030, 2060):
+        toks = (np.arange(n) * 7919 % 509).astype(np.int32)
+        want = prompt_logits(qb, m, toks, n + 1)[0]
+        assert np.isfinite(want).all() and want.std() > 0
+        for max_ctx in (4096, 8192, 8193, 40000):
+            assert np.array_equal(prompt_logits(qb, m, toks, max_ctx)[0], want), (n, max_ctx)
+    m.close()
