@@ -364,6 +364,37 @@ uint32_t qb_env_u32(const char *name, uint32_t dflt) {
     return (v && *v) ? (uint32_t)strtoul(v, nullptr, 10) : dflt;
 }
 
+// Decode attention of a qwen35 batch: kernel and split size.
+static void attention_form(qb_batch *b) {
+    const qb_model_config &c = b->m->cfg;
+    // The tensor-memory attention kernel wins once a call has enough keys to fill the GPU (one long context, or many
+    // sequences) and costs a few microseconds per call below that; the two kernels differ in the last bits, so the choice
+    // is a property of the batch (the keys it can hold), the same for every row the batch ever computes.
+    b->attn_tc = (uint64_t)b->n_seqs * b->max_ctx >= qb_env_u32("QW3B200_ATTN_TC_MIN_KEYS", 16384);
+    // Splits of 256 keys where the tensor-memory kernel runs (its tile pair); 128 keys otherwise: a short context then
+    // spreads over twice the SMs, each streaming half the K/V bytes (7.87 against 8.01 ms per step at 2 K context).
+    {
+        const bool tc_shape = (c.head_dim == 256 || c.head_dim == 128) && b->page_size == 16 && c.n_heads / std::max(1u, c.n_kv_heads) <= 8;
+        b->attn_split = b->attn_tc && tc_shape ? 256 : qb_env_u32("QW3B200_ATTN_SPLIT_SMALL", 128);
+        if (b->attn_split < 64 || b->attn_split % 64) b->attn_split = 128;
+    }
+}
+
+// Rows of a qwen35 prompt pass: 512, doubled up to 2048 while the context has use for them (fewer half-empty waves of GEMM tiles and
+// fewer launches: 2048 tokens of the 27B shape in passes of 512 / 1024 / 2048: 391 / 378 / 372 ms) and the split partials of attention
+// (rows x splits x heads x head size floats) stay below what 512 rows take at a context of 32768 in 256-key splits, with a few splits to
+// spare: 1.7 GB on that shape.  The other buffers of a row are 0.4 MB there (a pass of 2048 rows: 0.8 GB, of 512: 0.2).  A shard keeps 512:
+// its peers' receive areas are made for it.
+static constexpr size_t PASS_ROW_SPLITS = 68 * 1024;
+static uint32_t qwen35_pass_rows(qb_batch *b) {
+    attention_form(b);
+    uint32_t rows = b->m->arch->chunk;
+    if (b->m->tp_world != 1) return rows;
+    const size_t splits = ((size_t)b->max_ctx + b->k + 1) / b->attn_split + 1;
+    while (rows < 2048 && rows < b->max_ctx && 2 * rows * splits <= PASS_ROW_SPLITS) rows *= 2;
+    return rows;
+}
+
 // Caches, recurrent state and activations of the qwen35 family.
 static int qwen35_batch_alloc(qb_ctx *ctx, qb_batch *b, size_t slots) {
     qb_model *m = b->m;
@@ -371,17 +402,7 @@ static int qwen35_batch_alloc(qb_ctx *ctx, qb_batch *b, size_t slots) {
     const uint32_t n_seqs = b->n_seqs, max_ctx = b->max_ctx, draft_k = b->k, page_size = b->page_size;
     const uint32_t H = c.n_embd, K1 = draft_k + 1, L = c.n_layers, rows = b->rows_cap;
     b->gemm_impl = (int)qb_env_u32("QW3B200_GEMM_IMPL", 0);
-    // The tensor-memory attention kernel wins once a call has enough keys to fill the GPU (one long context, or many
-    // sequences) and costs a few microseconds per call below that; the two kernels differ in the last bits, so the choice
-    // is a property of the batch (the keys it can hold), the same for every row the batch ever computes.
-    b->attn_tc = (uint64_t)n_seqs * max_ctx >= qb_env_u32("QW3B200_ATTN_TC_MIN_KEYS", 16384);
-    // Splits of 256 keys where the tensor-memory kernel runs (its tile pair); 128 keys otherwise: a short context then
-    // spreads over twice the SMs, each streaming half the K/V bytes (7.87 against 8.01 ms per step at 2 K context).
-    {
-        const bool tc_shape = (c.head_dim == 256 || c.head_dim == 128) && page_size == 16 && c.n_heads / std::max(1u, c.n_kv_heads) <= 8;
-        b->attn_split = b->attn_tc && tc_shape ? 256 : qb_env_u32("QW3B200_ATTN_SPLIT_SMALL", 128);
-        if (b->attn_split < 64 || b->attn_split % 64) b->attn_split = 128;
-    }
+    attention_form(b);
     const uint32_t kvd = m->kvd();
     b->kc.assign(L + 1, nullptr); b->vc.assign(L + 1, nullptr); b->state.assign(L, nullptr); b->conv.assign(L, nullptr); b->conv_alt.assign(L, nullptr);
     for (uint32_t il = 0; il <= L; ++il) {
@@ -451,26 +472,12 @@ static void qwen35_batch_free(qb_batch *b) {
 
 extern "C" void qb_batch_destroy(qb_ctx *ctx, qb_batch *b);
 
-static int batch_create(qb_ctx *ctx, qb_model *m, uint32_t n_seqs, uint32_t max_ctx, uint32_t draft_k,
-                        uint32_t page_size, int page_order, uint32_t pool_pages, qb_batch **out) {
-    QB_REQUIRE(ctx && m && out && n_seqs > 0 && max_ctx > 0 && page_size > 0, "qb_batch_create: bad arguments");
-    QB_REQUIRE(draft_k <= 7, "draft depth %u unsupported (<= 7)", draft_k);
-    QB_REQUIRE(draft_k == 0 || m->cfg.mtp_layers == 1, "draft depth > 0 needs the MTP layer");
-    QB_CUDA(cudaSetDevice(ctx->device));
+// Everything a batch holds, for prompt passes of b->chunk rows; b's capacity is set.  What a failure leaves is the caller's to free.
+static int batch_fill(qb_ctx *ctx, qb_batch *b, int page_order, uint32_t pool_pages) {
+    qb_model *m = b->m;
     const qb_model_config &c = m->cfg;
-    qb_batch *b = new qb_batch();
-    b->m = m; b->n_seqs = n_seqs; b->n_active = n_seqs; b->max_ctx = max_ctx; b->k = draft_k; b->page_size = page_size;
+    const uint32_t n_seqs = b->n_seqs, max_ctx = b->max_ctx, draft_k = b->k, page_size = b->page_size;
     b->pages_per_seq = (max_ctx + draft_k + 1 + page_size - 1) / page_size;
-    // Rows of an ingestion pass: the family's, doubled up to 2048 while the context has use for them (fewer half-empty waves of
-    // GEMM tiles and fewer launches: 2048 tokens in passes of 512 / 1024 / 2048: 391 / 378 / 372 ms on the 27B shape; of 1024 / 2048:
-    // 10.1 / 9.4 and 13.0 / 11.7 ms on the layered models) and, for the hybrid, rows x context stays at what 512 rows take at 32768 (the
-    // attention's split partials grow with that product).  A layered model's rows depend on where its passes end (a pass of up to 64 rows
-    // takes split products, one of up to 16 the absorbed attention), so its size follows nothing but whether one pass holds the whole
-    // context: the same prompt gives the same bits at every max_ctx.  A shard keeps its size: its peers' receive areas are made for it.
-    uint32_t chunk = m->arch->chunk;
-    if (m->tp_world == 1)
-        while (chunk < 2048 && chunk < max_ctx && (m->layered || (size_t)2 * chunk * max_ctx <= (size_t)512 * 32768)) chunk *= 2;
-    b->chunk = std::max(1u, qb_env_u32("QW3B200_PREFILL_CHUNK", chunk));
     b->logit_rows = n_seqs * (draft_k + 1);
     b->rows_cap = std::max(b->chunk, b->logit_rows);
     const uint32_t H = c.n_embd, K1 = draft_k + 1, rows = b->rows_cap;
@@ -531,12 +538,33 @@ static int batch_create(qb_ctx *ctx, qb_model *m, uint32_t n_seqs, uint32_t max_
     QB_CUDA(cudaMalloc(&b->logits, (size_t)b->logit_rows * V * sizeof(float)));
     QB_CUDA(cudaMalloc(&b->am_val, (size_t)b->logit_rows * QB_ARGMAX_BLOCKS * sizeof(float)));
     QB_CUDA(cudaMalloc(&b->am_idx, (size_t)b->logit_rows * QB_ARGMAX_BLOCKS * sizeof(int32_t)));
-    if (const int st = m->arch->batch_alloc(ctx, b, slots); st != QB_OK) { qb_batch_destroy(ctx, b); return st; }
+    QB_TRY(m->arch->batch_alloc(ctx, b, slots));
     b->host_pos.assign(n_seqs, 0);
     b->chunk_end_pos.assign(n_seqs, -1);
     QB_CUDA(cudaStreamSynchronize(ctx->stream));
-    *out = b;
     return QB_OK;
+}
+
+static int batch_create(qb_ctx *ctx, qb_model *m, uint32_t n_seqs, uint32_t max_ctx, uint32_t draft_k,
+                        uint32_t page_size, int page_order, uint32_t pool_pages, qb_batch **out) {
+    QB_REQUIRE(ctx && m && out && n_seqs > 0 && max_ctx > 0 && page_size > 0, "qb_batch_create: bad arguments");
+    QB_REQUIRE(draft_k <= 7, "draft depth %u unsupported (<= 7)", draft_k);
+    QB_REQUIRE(draft_k == 0 || m->cfg.mtp_layers == 1, "draft depth > 0 needs the MTP layer");
+    QB_CUDA(cudaSetDevice(ctx->device));
+    const bool asked = getenv("QW3B200_PREFILL_CHUNK") && *getenv("QW3B200_PREFILL_CHUNK");
+    for (uint32_t chunk = asked ? std::max(1u, qb_env_u32("QW3B200_PREFILL_CHUNK", 0)) : 0;;) {
+        qb_batch *b = new qb_batch();
+        b->m = m; b->n_seqs = n_seqs; b->n_active = n_seqs; b->max_ctx = max_ctx; b->k = draft_k; b->page_size = page_size;
+        if (chunk == 0) chunk = m->arch->pass_rows(b);
+        b->chunk = chunk;
+        const int st = batch_fill(ctx, b, page_order, pool_pages);
+        if (st == QB_OK) { *out = b; return QB_OK; }
+        const bool memory = cudaGetLastError() == cudaErrorMemoryAllocation;
+        qb_batch_destroy(ctx, b);
+        // where the device has no room for the wide pass, the narrower ones, down to the family's own, give the same bits
+        if (!memory || asked || !m->arch->pass_free || chunk <= m->arch->chunk) return st;
+        chunk /= 2;
+    }
 }
 
 extern "C" int qb_batch_create(qb_ctx *ctx, qb_model *m, uint32_t n_seqs, uint32_t max_ctx, uint32_t draft_k,
@@ -926,7 +954,7 @@ static int qwen35_head(qb_ctx *ctx, qb_batch *b, const int32_t *row_map, uint32_
     return gemm_to(ctx, b, b->m->output, b->xq_h, rows, dst);
 }
 
-extern const QbArch ARCH_QWEN35 = {"qwen35", 512, qwen35_batch_alloc, qwen35_batch_free, qwen35_forward, qwen35_head, qwen35_model_free};
+extern const QbArch ARCH_QWEN35 = {"qwen35", 512, qwen35_pass_rows, true, qwen35_batch_alloc, qwen35_batch_free, qwen35_forward, qwen35_head, qwen35_model_free};
 
 // The model's layers on a row set.  tokens on the device ([rows]).  Leaves the pre-output-norm hidden rows
 // in b->hid[0 .. rows).  logits: 0 none, 1 every row, 2 last row of each sequence.

@@ -21,7 +21,10 @@ struct RowSet {
 // caches and activations for a batch, runs rows through its layers and turns hidden rows into logits.
 struct QbArch {
     const char *name;
-    uint32_t chunk;                      // rows of a prompt chunk
+    uint32_t chunk;                      // rows of a prompt pass, the family's own (a shard's, and the least a batch takes)
+    // Rows of a batch's prompt pass by its model and capacity (b->n_seqs, max_ctx, k, page_size are set).
+    uint32_t (*pass_rows)(qb_batch *b);
+    bool pass_free;                      // a row's bits do not depend on the pass it is in
     int (*batch_alloc)(qb_ctx *ctx, qb_batch *b, size_t slots);     // slots: K/V positions the paged caches hold
     void (*batch_free)(qb_batch *b);
     // Leaves the residual rows in b->hid[0 .. rows).  checkpoints: keep the recurrent state after every row (verify rows).

@@ -717,7 +717,13 @@ int layered_head(qb_ctx *ctx, qb_batch *b, const int32_t *row_map, uint32_t rows
     return qb_dense_gemm(ctx, Y.head, B->x, rows, dst, 1);
 }
 
-const QbArch ARCH_LAYERED = {"layered", 1024, layered_batch_alloc, layered_batch_free, layered_forward, layered_head, layered_model_free};
+// Rows of a prompt pass: 2048 (in passes of 1024 / 2048 2048 tokens took 10.1 / 9.4 ms on the latent-attention family and 13.0 / 11.7 on the
+// shared-key/value one), or the family's 1024 where one such pass holds the whole context.  Rows depend on where passes end (a pass of up
+// to 64 rows takes split products, one of up to 16 the absorbed attention), so the size follows nothing else: the same prompt
+// gives the same bits at every max_ctx, and a batch that does not fit is refused, not cut.
+uint32_t layered_pass_rows(qb_batch *b) { return b->max_ctx > 1024 ? 2048 : 1024; }
+
+const QbArch ARCH_LAYERED = {"layered", 1024, layered_pass_rows, false, layered_batch_alloc, layered_batch_free, layered_forward, layered_head, layered_model_free};
 
 int layered_create(qb_ctx *ctx, const std::string &config, bool f32, Source &src, qb_model **out) {
     auto Y = std::make_unique<QbLayered>();

@@ -168,3 +168,38 @@ def test_layered_prompt_does_not_depend_on_the_capacity(qb, ctx, family, dtype):
         for max_ctx in (4096, 8192, 8193, 40000):
             assert np.array_equal(prompt_logits(qb, m, toks, max_ctx)[0], want), (n, max_ctx)
     m.close()
+
+
+def test_hybrid_pass_keeps_its_memory_bounded_and_shrinks_where_there_is_none(qb, ctx, monkeypatch):
+    """Rows x attention splits of a prompt pass are bounded whatever the context, and a batch that does not fit with the wide pass is
+    created with a narrower one: the same logits."""
+    m = qb.Model(ctx, qb.configs.tiny(), 5)
+    toks = (np.arange(700) * 7919 % 4093).astype(np.int32)
+    for max_ctx, rows in ((500, 512), (1000, 1024), (2056, 2048), (4096, 2048), (8192, 1024), (30000, 512)):
+        got = prompt_logits(qb, m, toks[:400], max_ctx)[1]
+        assert got == rows and got * (max_ctx // 128 + 1) <= max(68 * 1024, 512 * (max_ctx // 128 + 1)), max_ctx
+
+    def held(max_ctx):
+        """Device bytes that a batch takes."""
+        ctx.sync()
+        free = ctx.mem_info()[0]
+        b = qb.Batch(m, 1, max_ctx, 0)
+        ctx.sync()
+        used = free - ctx.mem_info()[0]
+        b.close()
+        return used
+
+    want, rows = prompt_logits(qb, m, toks, 4000)
+    wide = held(4000)
+    monkeypatch.setenv("QW3B200_PREFILL_CHUNK", "512")
+    narrow = held(4000)
+    monkeypatch.delenv("QW3B200_PREFILL_CHUNK")
+    assert rows == 2048 and wide > narrow + (32 << 20)
+    ctx.sync()
+    filler = ctx.empty(ctx.mem_info()[0] - (wide + narrow) // 2, np.uint8)
+    try:
+        got, rows = prompt_logits(qb, m, toks, 4000)
+    finally:
+        filler.free()
+    assert rows in (512, 1024) and np.array_equal(got, want)
+    m.close()
