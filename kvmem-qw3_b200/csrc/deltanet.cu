@@ -26,7 +26,9 @@ namespace {
 //   columns (= one quantisation block).
 // The q/k conv windows are read by several CTAs but written by one (v head < nk, column block 0), so the kernel
 // reads the conv state from conv and writes it to conv_out (a different buffer: the caller ping-pongs).
-// RB = rows per block (one conv / norm phase, one exchange of the head's sums of squares and one norm-gate phase per block).
+// RB = rows per block (one conv / norm phase, one exchange of the head's sums of squares and one norm-gate phase per block): 4 for
+// the decode and verify steps, 8 where 16 rows or more per sequence keep a checkpoint each and the per-block costs dominate (48 heads of
+// 128, one sequence: 16 rows 35.4 us with 4-row blocks, 29.1 with 8; 64 rows 139.8 and 102.8).  A row's arithmetic does not depend on RB.
 template <int HD, int CPW, int RB, int MINB>
 __global__ void __launch_bounds__(512, MINB) dn_fused_kernel(DnArgs a) {
     constexpr int COLS = 16 * CPW, NCB = HD / COLS, NQB = COLS / 32, RPL = HD / 32, NCH = 2 * HD + COLS;
@@ -58,33 +60,67 @@ __global__ void __launch_bounds__(512, MINB) dn_fused_kernel(DnArgs a) {
     // The inputs of a row block (projection rows, gate inputs, z) do not depend on the state slot: they are
     // requested first, and the next block's while the current one is processed.
     struct BlockIn { float cur[RB]; float zv, graw; };
+    // 8-row form: every load of a block is issued before the first add (a load-add-load-add chain exposes one memory
+    // latency per row); each element still adds its K-segment partials in ascending order.
     auto load_block = [&](uint32_t rb0) {
         BlockIn in;
         const uint32_t nrows = rb0 < R ? min((uint32_t)RB, R - rb0) : 0u;
         const size_t row0 = (size_t)seq * R + rb0;
-        if (a.proj_S == 2) {                      // the usual split of the input projection: both partials of every row first
-            float p1[RB];
+        if constexpr (RB <= 4) {
+            // the step forms (64 registers per thread): element by element
+            if (a.proj_S == 2) {                      // the usual split of the input projection: both partials of every row first
+                float p1[RB];
 #pragma unroll
-            for (int t = 0; t < RB; ++t) {
-                const bool on = has && (uint32_t)t < nrows;
-                in.cur[t] = on ? a.proj[(row0 + t) * a.proj_stride + ch] : 0.0f;
-                p1[t] = on ? a.proj[(row0 + t) * a.proj_stride + ch + a.proj_pstride] : 0.0f;
+                for (int t = 0; t < RB; ++t) {
+                    const bool on = has && (uint32_t)t < nrows;
+                    in.cur[t] = on ? a.proj[(row0 + t) * a.proj_stride + ch] : 0.0f;
+                    p1[t] = on ? a.proj[(row0 + t) * a.proj_stride + ch + a.proj_pstride] : 0.0f;
+                }
+#pragma unroll
+                for (int t = 0; t < RB; ++t) in.cur[t] += p1[t];
+            } else {
+#pragma unroll
+                for (int t = 0; t < RB; ++t) {
+                    in.cur[t] = 0.0f;
+                    if (has && (uint32_t)t < nrows) in.cur[t] = qb_ldsum(a.proj, (row0 + t) * a.proj_stride + ch, a.proj_S, a.proj_pstride);
+                }
             }
-#pragma unroll
-            for (int t = 0; t < RB; ++t) in.cur[t] += p1[t];
-        } else {
-#pragma unroll
-            for (int t = 0; t < RB; ++t) {
-                in.cur[t] = 0.0f;
-                if (has && (uint32_t)t < nrows) in.cur[t] = qb_ldsum(a.proj, (row0 + t) * a.proj_stride + ch, a.proj_S, a.proj_pstride);
-            }
+            in.zv = 0.0f;
+            if (ng_q < NQB && ng_t < nrows)
+                in.zv = qb_ldsum(a.proj, (row0 + ng_t) * a.proj_stride + C + vh * HD + cb * COLS + ng_q * 32 + lane, a.proj_S, a.proj_pstride);
+            in.graw = 0.0f;
+            if (warp == 15 && lane < 2 * nrows)      // (row, decay | write strength) of the block: lanes of the last warp
+                in.graw = qb_ldsum(a.proj, (row0 + (lane >> 1)) * a.proj_stride + C + vdim + (lane & 1) * a.nv + vh, a.proj_S, a.proj_pstride);
+            return in;
         }
-        in.zv = 0.0f;
-        if (ng_q < NQB && ng_t < nrows)
-            in.zv = qb_ldsum(a.proj, (row0 + ng_t) * a.proj_stride + C + vh * HD + cb * COLS + ng_q * 32 + lane, a.proj_S, a.proj_pstride);
-        in.graw = 0.0f;
-        if (warp == 15 && lane < 2 * nrows)      // (row, decay | write strength) of the block: lanes of the last warp
-            in.graw = qb_ldsum(a.proj, (row0 + (lane >> 1)) * a.proj_stride + C + vdim + (lane & 1) * a.nv + vh, a.proj_S, a.proj_pstride);
+        const uint32_t S = a.proj_S;
+        const bool two = S > 1;
+        const bool hz = ng_q < NQB && ng_t < nrows, hg = warp == 15 && lane < 2 * nrows;
+        const size_t iz = (row0 + ng_t) * a.proj_stride + C + vh * HD + cb * COLS + ng_q * 32 + lane;
+        const size_t ig = (row0 + (lane >> 1)) * a.proj_stride + C + vdim + (lane & 1) * a.nv + vh;
+        float p0[RB], p1[RB];
+#pragma unroll
+        for (int t = 0; t < RB; ++t) {
+            const bool on = has && (uint32_t)t < nrows;
+            p0[t] = on ? a.proj[(row0 + t) * a.proj_stride + ch] : 0.0f;
+            p1[t] = on && two ? a.proj[(row0 + t) * a.proj_stride + ch + a.proj_pstride] : 0.0f;
+        }
+        const float z0 = hz ? a.proj[iz] : 0.0f, z1 = hz && two ? a.proj[iz + a.proj_pstride] : 0.0f;
+        const float g0 = hg ? a.proj[ig] : 0.0f, g1 = hg && two ? a.proj[ig + a.proj_pstride] : 0.0f;
+#pragma unroll
+        for (int t = 0; t < RB; ++t) in.cur[t] = two ? p0[t] + p1[t] : p0[t];
+        in.zv = two ? z0 + z1 : z0;
+        in.graw = two ? g0 + g1 : g0;
+        for (uint32_t sg = 2; sg < S; ++sg) {                 // further segments: again all loads, then the adds
+            const size_t off = (size_t)sg * a.proj_pstride;
+#pragma unroll
+            for (int t = 0; t < RB; ++t) p0[t] = has && (uint32_t)t < nrows ? a.proj[(row0 + t) * a.proj_stride + ch + off] : 0.0f;
+            const float zs = hz ? a.proj[iz + off] : 0.0f, gs = hg ? a.proj[ig + off] : 0.0f;
+#pragma unroll
+            for (int t = 0; t < RB; ++t) in.cur[t] += p0[t];
+            in.zv += zs;
+            in.graw += gs;
+        }
         return in;
     };
     BlockIn nxt = load_block(0);
@@ -651,10 +687,10 @@ int qb_launch_deltanet(qb_ctx *ctx, const DnArgs &a) {
     QB_REQUIRE(a.conv_out && a.conv_out != a.conv, "deltanet: the new conv state needs a buffer of its own");
     // one request: 32 state columns per CTA (more CTAs, shortest critical path); several: 64 per CTA (the per-CTA
     // work that does not depend on the column count — the head's q/k conv, the barriers — is paid half as often)
-    // prompt ingestion (16 rows or more per sequence, only the last state kept): the three-launch form.  Below 16 rows its two more
-    // launches cost what the shorter rows give.
-    const bool wide = a.n_seqs > 2, many = a.rows_per_seq >= 16 && !a.write_all;
-    if (a.hd == 128) return many ? launch_ingest<128>(ctx, a) : wide ? launch_fused<128, 4, 4, 2>(ctx, a) : launch_fused<128, 2, 4, 2>(ctx, a);
-    if (a.hd == 64) return many ? launch_ingest<64>(ctx, a) : wide ? launch_fused<64, 4, 4, 2>(ctx, a) : launch_fused<64, 2, 4, 2>(ctx, a);
+    // 16 rows or more per sequence: the three-launch form where only the last state is kept (prompt ingestion; below 16 rows its two more
+    // launches cost what the shorter rows give), 64 columns per CTA and 8-row blocks where every row leaves a checkpoint
+    const bool wide = a.n_seqs > 2, many = a.rows_per_seq >= 16, ingest = many && !a.write_all;
+    if (a.hd == 128) return ingest ? launch_ingest<128>(ctx, a) : many ? launch_fused<128, 4, 8, 1>(ctx, a) : wide ? launch_fused<128, 4, 4, 2>(ctx, a) : launch_fused<128, 2, 4, 2>(ctx, a);
+    if (a.hd == 64) return ingest ? launch_ingest<64>(ctx, a) : many ? launch_fused<64, 4, 8, 1>(ctx, a) : wide ? launch_fused<64, 4, 4, 2>(ctx, a) : launch_fused<64, 2, 4, 2>(ctx, a);
     return qb_fail(QB_ERR_UNSUPPORTED, "deltanet: head dim %u unsupported (64/128)", a.hd);
 }

@@ -44,6 +44,40 @@ def test_deltanet_prompt_rows_equal_the_same_rows_in_small_parts(qb, ctx, nk, nv
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("nk,nv,hd,n_seqs,R", [(2, 6, 128, 1, 16), (2, 4, 128, 3, 17), (1, 2, 64, 2, 23), (2, 4, 64, 1, 33)])
+def test_deltanet_checkpoints_of_many_rows_equal_single_rows(qb, ctx, nk, nv, hd, n_seqs, R):
+    """With checkpoints, 16 rows and more take 8-row blocks: outputs, and the state and conv window after every row, equal those of
+    one row at a time, bit for bit."""
+    rng = np.random.default_rng(R + hd)
+    Cq = (2 * nk + nv) * hd
+    stride = Cq + nv * hd + 2 * nv
+    proj = rng.standard_normal((n_seqs, R, stride)).astype(np.float32)
+    state = (rng.standard_normal((n_seqs, R, nv, hd, hd)) * 0.05).astype(np.float32)
+    conv = rng.standard_normal((n_seqs, R, Cq, 3)).astype(np.float32)
+    cw = ctx.array(rng.uniform(-0.5, 0.5, (Cq, 4)).astype(np.float32))
+    sa = ctx.array((-np.exp(rng.uniform(0, np.log(16), nv))).astype(np.float32))
+    dt = ctx.array(rng.uniform(-4, -1, nv).astype(np.float32))
+    nw = ctx.array(rng.uniform(0.5, 1.5, hd).astype(np.float32))
+    slot = rng.integers(0, R, n_seqs).astype(np.int32)
+
+    def call(rows, d_state, d_conv, slots, slot_in, write_all):
+        n = rows.shape[1]
+        core = ctx.empty((n_seqs, n, nv * hd), np.float32)
+        qb.binding.check(qb.lib().qb_deltanet_rows(ctx.h, ctx.array(np.ascontiguousarray(rows)).ptr, n_seqs, n, stride, cw.ptr, sa.ptr, dt.ptr,
+                                                   nw.ptr, nk, nv, hd, C.c_float(1e-6), d_state.ptr, d_conv.ptr, slots, ctx.array(slot_in).ptr,
+                                                   write_all, core.ptr))
+        return core.download()
+
+    d_state, d_conv = ctx.array(state), ctx.array(conv)
+    core = call(proj, d_state, d_conv, R, slot, 1)
+    states, convs = d_state.download(), d_conv.download()
+    pick = np.arange(n_seqs), slot
+    d_state, d_conv = ctx.array(state[pick][:, None]), ctx.array(conv[pick][:, None])
+    for t in range(R):
+        assert np.array_equal(call(proj[:, t:t + 1], d_state, d_conv, 1, np.zeros(n_seqs, np.int32), 0)[:, 0], core[:, t]), t
+        assert np.array_equal(d_state.download()[:, 0], states[:, t]) and np.array_equal(d_conv.download()[:, 0], convs[:, t]), t
+
+
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64, 65, 100])
 @pytest.mark.parametrize("N,K,stride", [(64, 32, 32), (130, 100, 101), (9600, 64, 68), (200, 2056, 2056)])
 def test_dense_product_in_32_bits(qb, ctx, M, N, K, stride):
