@@ -487,11 +487,16 @@ __global__ void __launch_bounds__(1024) attn_merge_kernel(AttnArgs a, const int3
     }
 }
 
-// The same merge for up to 32 splits: four consecutive values a thread, hd / 4 threads a (row, head), weights recomputed by each thread instead
-// of passed through shared memory -- no barrier and no idle group; the same sums in the same order.  A prompt pass of 2048 rows x 24 heads
-// of 256 with up to 9 splits: 500 -> 188 us; 128 rows 14.2 -> 7.7; bound by reading the partials.  Under 64 rows the chain over the splits is
-// the longer one (4 rows, 17 splits: 8.8 against 5.7).
-constexpr uint32_t MERGE4_SPLITS = 32, MERGE4_THREADS = 256, MERGE4_MIN_ROWS = 64;
+// The same merge for launches that fill the GPU: four consecutive values a thread, hd / 4 threads a (row, head), weights recomputed by each
+// thread instead of passed through shared memory -- no barrier and no idle group; the same sums in the same order.  Bound by reading
+// the partials.  A prompt pass of 2048 rows x 24 heads of 256 with up to 17 splits: 741 -> 178 us; 128 rows of 24 heads 24 -> 13.
+// The line lies where its chains over the splits stop being hidden by other CTAs (call with both attention launches, us, this form last):
+// 256 CTAs (8 heads of 256, 128 rows): 4 splits 20.4 / 17.9, 33 splits 68 / 54, 129 splits 226 / 218, 257 splits 413 / 420; 128 CTAs (64 rows):
+// 9 splits 18.4 / 18.8, 33 splits 38.7 / 36.6, 65 splits 61 / 63; 64 CTAs (32 rows): 9 splits 18.2 / 18.1, 17 splits 18.3 / 21.4.
+// Heads of 64 and 128 from 17 splits or 2048 CTAs on (16 heads of 128: 256 rows, 17 splits 107 / 98; 1024 rows, 9 splits 128 / 104): below, its
+// CTAs, launched early, wait on the SMs beside the split kernel's and the call takes longer although the merge does not (256 rows, 7 splits:
+// 42 / 53, the merge alone 18 / 14).
+constexpr uint32_t MERGE4_THREADS = 256, MERGE4_MIN_CTAS = 256, MERGE4_MAX_SPLITS = 128, MERGE4_NARROW_SPLITS = 17, MERGE4_NARROW_CTAS = 2048;
 __global__ void __launch_bounds__(MERGE4_THREADS) attn_merge4_kernel(AttnArgs a, const int32_t *__restrict__ seq_pos, uint32_t R, uint32_t max_splits,
                                                                      float *out, int8_t *q8, uint32_t q_pitch, float *dsc, uint32_t d_ld) {
     QB_PDL_ENTER();
@@ -559,9 +564,10 @@ static int launch_merge(qb_ctx *ctx, const AttnArgs &aa, const int32_t *seq_pos,
                         uint32_t q_pitch, float *d, uint32_t d_ld) {
     const bool vec = ((uintptr_t)aa.qkv & 15) == 0 && aa.row_stride % 4 == 0 && aa.in_pstride % 4 == 0 && ((uintptr_t)aa.part_acc & 15) == 0 && ((uintptr_t)aa.part_ml & 7) == 0 &&
                      ((uintptr_t)out & 15) == 0 && ((uintptr_t)q8 & 3) == 0 && q_pitch % 4 == 0;
-    if (vec && aa.rows >= MERGE4_MIN_ROWS && ms <= MERGE4_SPLITS && aa.hd % 32 == 0 && aa.hd <= 4 * MERGE4_THREADS && MERGE4_THREADS % (aa.hd / 4) == 0) {
-        const uint32_t per_cta = MERGE4_THREADS / (aa.hd / 4);
-        QB_CUDA(qb_launch_pdl(ctx->stream, attn_merge4_kernel, dim3((aa.rows * aa.n_heads + per_cta - 1) / per_cta), dim3(MERGE4_THREADS), (size_t)0, aa, seq_pos, R, ms, out, q8,
+    const uint32_t per_cta = aa.hd % 32 == 0 && aa.hd <= 4 * MERGE4_THREADS && MERGE4_THREADS % (aa.hd / 4) == 0 ? MERGE4_THREADS / (aa.hd / 4) : 0;
+    const uint32_t ctas = per_cta ? (aa.rows * aa.n_heads + per_cta - 1) / per_cta : 0;
+    if (vec && ctas >= MERGE4_MIN_CTAS && ms <= MERGE4_MAX_SPLITS && (aa.hd >= 256 || ms >= MERGE4_NARROW_SPLITS || ctas >= MERGE4_NARROW_CTAS)) {
+        QB_CUDA(qb_launch_pdl(ctx->stream, attn_merge4_kernel, dim3(ctas), dim3(MERGE4_THREADS), (size_t)0, aa, seq_pos, R, ms, out, q8,
                               q_pitch, d, d_ld));
         QB_LAUNCHED(ctx, "attn_merge_kernel");
         return QB_OK;

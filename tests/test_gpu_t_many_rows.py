@@ -179,6 +179,35 @@ def test_merge_of_many_rows_equals_few_rows(qb, ctx, monkeypatch, rows, pos, hea
     np.testing.assert_array_equal(whole, parts)
 
 
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("rows,pos,heads,kv,hd", [(257, 0, 4, 2, 256), (79, 3, 13, 13, 256), (1025, 0, 1, 1, 256), (128, 4080, 8, 1, 256), (130, 8300, 8, 1, 256),
+                                                  (256, 32200, 4, 1, 256), (257, 4300, 8, 2, 128), (515, 4100, 8, 2, 64), (1025, 0, 16, 4, 128), (127, 100, 8, 2, 256),
+                                                  (256, 33000, 4, 1, 256)])
+def test_merge_that_fills_the_gpu_equals_small_ones(qb, ctx, rows, pos, heads, kv, hd, gated):
+    """256 CTAs and more of the barrier-free merge (one to 128 splits of 256 keys, units that do not fill the last CTA), and the
+    launches just outside its rule, against parts of 16 rows."""
+    rng = np.random.default_rng(rows + pos)
+    page, n_pages = 16, (pos + rows + 15) // 16
+    stride = 2 * heads * hd + 2 * kv * hd
+    qkv = rng.standard_normal((rows, stride), dtype=np.float32)
+    k = ctx.array((rng.standard_normal((n_pages * page, kv, hd), dtype=np.float32) * np.float32(0.3)).astype(np.float16))
+    v = ctx.array(rng.standard_normal((n_pages * page, kv, hd), dtype=np.float32).astype(np.float16))
+    table = ctx.array(np.arange(n_pages, dtype=np.int32)[None])
+    L = qb.lib()
+    call = L.qb_attention_paged_gated if gated else L.qb_attention_paged
+
+    def run(lo, hi):
+        out = ctx.empty((hi - lo, heads * hd), np.float32)
+        qb.binding.check(call(ctx.h, ctx.array(qkv[lo:hi]).ptr, hi - lo, stride, heads, kv, hd, ctx.array(np.array([pos + lo], np.int32)).ptr, 1, table.ptr,
+                              n_pages, page, k.ptr, v.ptr, pos + rows, out.ptr))
+        return out.download()
+
+    whole = run(0, rows)
+    assert np.isfinite(whole).all()
+    for lo in list(range(0, rows, 16))[::3] + [rows - 16]:
+        np.testing.assert_array_equal(whole[lo:lo + 16], run(lo, min(lo + 16, rows)))
+
+
 def prompt_logits(qb, model, toks, max_ctx):
     b = qb.Batch(model, 1, max_ctx, 0)
     b.prefill(0, toks)
