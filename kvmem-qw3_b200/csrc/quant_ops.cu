@@ -180,10 +180,16 @@ __global__ void __launch_bounds__(NQ_THREADS) norm_quant_kernel(NormQuantArgs a,
     if (!a.w) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // complete the opening arrive
 }
 
-// From 256 rows on (up to 8192 elements each): one CTA per row, no cluster -- with rows enough for every SM the eight-fold split only
-// multiplies barriers (2048 rows of 5120 with six or seven partial sums: 140 -> 104 us; at 128 rows it is the slower one, 11.0 against 6.6).  A thread stands for the thread of the same index in four of the eight
-// CTAs of norm_quant_kernel, so every sum is formed from the same parts in the same order.
+// Many rows of up to 8192 elements: one CTA per row, no cluster -- with rows enough for every SM the eight-fold split only multiplies
+// barriers.  A thread stands for the thread of the same index in four of the eight CTAs of norm_quant_kernel, so every sum is formed from the same parts in
+// the same order.  Two CTAs fit an SM.  Cluster form / this one, us: plain norm of 5120, 256 rows 8.0 / 4.9, 300 rows 9.4 / 7.9, 2048 rows 57 / 29;
+// quantiser alone 256 rows 5.8 / 4.8, 300 rows 6.6 / 7.5, 331 rows 7.0 / 7.7, 400 rows 8.1 / 7.8; norm of up to seven partial sums (between events) 256
+// rows 17.9 / 15.3, 300 rows 21.2 / 22.0, 331 rows 21.7 / 23.2, 400 rows 25.9 / 25.0, 2048 rows 102 / 81: where a row's loads and not its
+// barriers take the time, a second wave of CTAs has to be a third full.
 constexpr uint32_t NQR_THREADS = 512, NQR_MIN_ROWS = 256;
+static bool nq_takes_rows(const NormQuantArgs &a, uint32_t sms) {
+    return a.M >= NQR_MIN_ROWS && ((a.w && a.S == 0) || a.M <= 2 * sms || a.M >= 8 * sms / 3);
+}
 __global__ void __launch_bounds__(NQR_THREADS, 2) norm_quant_rows_kernel(NormQuantArgs a, uint32_t vec) {
     QB_PDL_ENTER();
     __shared__ float red[NQ_CLUSTER][NQ_THREADS / 32];
@@ -251,7 +257,7 @@ int qb_launch_norm_quant(qb_ctx *ctx, const NormQuantArgs &a) {
                a.q_pitch % 4 == 0 && a.q_col_off % 4 == 0, "norm_quant: gain / output buffers must be 16-byte aligned");
     auto al = [](const void *p, size_t stride) { return ((uintptr_t)p & 15) == 0 && stride % 4 == 0; };
     const uint32_t vec = (al(a.x, a.x_stride) ? 1u : 0u) | (al(a.parts, a.part_ld) ? 2u : 0u) | (al(a.h_out, a.h_stride) ? 4u : 0u);
-    if (per <= 32 && a.M >= NQR_MIN_ROWS) QB_CUDA(qb_launch_pdl(ctx->stream, norm_quant_rows_kernel, dim3(a.M), dim3(NQR_THREADS), (size_t)0, a, vec));
+    if (per <= 32 && nq_takes_rows(a, (uint32_t)ctx->sm_count)) QB_CUDA(qb_launch_pdl(ctx->stream, norm_quant_rows_kernel, dim3(a.M), dim3(NQR_THREADS), (size_t)0, a, vec));
     else if (per <= 32) QB_CUDA(launch_norm_quant<1>(ctx->stream, a, vec));
     else if (per <= 64) QB_CUDA(launch_norm_quant<2>(ctx->stream, a, vec));
     else QB_CUDA(launch_norm_quant<4>(ctx->stream, a, vec));

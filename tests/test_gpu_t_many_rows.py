@@ -132,6 +132,12 @@ def test_norm_and_quantiser_of_many_rows_equal_few_rows(qb, ctx, M, n):
     assert np.array_equal(q, np.concatenate([p[0] for p in parts])) and np.array_equal(d, np.concatenate([p[1] for p in parts], 1))
 
 
+@pytest.mark.parametrize("waves", [(2, 0), (2, 1), (8 / 3, -1), (8 / 3, 0), (8 / 3, 1), (5, 3)])
+def test_norm_and_quantiser_around_a_second_wave(qb, ctx, waves):
+    """The quantiser's one-CTA form stops past two rows per SM and starts again at 8/3 of them: the same bits on either side."""
+    test_norm_and_quantiser_of_many_rows_equal_few_rows(qb, ctx, int(waves[0] * ctx.sm_count) + waves[1], 1056)
+
+
 @pytest.mark.parametrize("M", [16, 17, 65, 130])
 def test_feed_forward_input_of_many_rows_equals_one_launch_form(qb, orc, ctx, M):
     """silu(gate) * up quantised by the vectorised kernel (any rows) == the GEMM's own epilogue (up to 16 rows at a time)."""
