@@ -569,7 +569,7 @@ static int launch_merge(qb_ctx *ctx, const AttnArgs &aa, const int32_t *seq_pos,
     if (vec && ctas >= MERGE4_MIN_CTAS && ms <= MERGE4_MAX_SPLITS && (aa.hd >= 256 || ms >= MERGE4_NARROW_SPLITS || ctas >= MERGE4_NARROW_CTAS)) {
         QB_CUDA(qb_launch_pdl(ctx->stream, attn_merge4_kernel, dim3(ctas), dim3(MERGE4_THREADS), (size_t)0, aa, seq_pos, R, ms, out, q8,
                               q_pitch, d, d_ld));
-        QB_LAUNCHED(ctx, "attn_merge_kernel");
+        QB_LAUNCHED(ctx, "attn_merge4_kernel");
         return QB_OK;
     }
     const uint32_t nb_max = (ms + MERGE_BLOCK - 1) / MERGE_BLOCK;

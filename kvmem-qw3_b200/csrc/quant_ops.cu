@@ -257,8 +257,12 @@ int qb_launch_norm_quant(qb_ctx *ctx, const NormQuantArgs &a) {
                a.q_pitch % 4 == 0 && a.q_col_off % 4 == 0, "norm_quant: gain / output buffers must be 16-byte aligned");
     auto al = [](const void *p, size_t stride) { return ((uintptr_t)p & 15) == 0 && stride % 4 == 0; };
     const uint32_t vec = (al(a.x, a.x_stride) ? 1u : 0u) | (al(a.parts, a.part_ld) ? 2u : 0u) | (al(a.h_out, a.h_stride) ? 4u : 0u);
-    if (per <= 32 && nq_takes_rows(a, (uint32_t)ctx->sm_count)) QB_CUDA(qb_launch_pdl(ctx->stream, norm_quant_rows_kernel, dim3(a.M), dim3(NQR_THREADS), (size_t)0, a, vec));
-    else if (per <= 32) QB_CUDA(launch_norm_quant<1>(ctx->stream, a, vec));
+    if (per <= 32 && nq_takes_rows(a, (uint32_t)ctx->sm_count)) {
+        QB_CUDA(qb_launch_pdl(ctx->stream, norm_quant_rows_kernel, dim3(a.M), dim3(NQR_THREADS), (size_t)0, a, vec));
+        QB_LAUNCHED(ctx, "norm_quant_rows_kernel");
+        return QB_OK;
+    }
+    if (per <= 32) QB_CUDA(launch_norm_quant<1>(ctx->stream, a, vec));
     else if (per <= 64) QB_CUDA(launch_norm_quant<2>(ctx->stream, a, vec));
     else QB_CUDA(launch_norm_quant<4>(ctx->stream, a, vec));
     QB_LAUNCHED(ctx, "norm_quant_kernel");
@@ -331,12 +335,14 @@ int qb_launch_swiglu_quant(qb_ctx *ctx, const float *gu, uint32_t gu_stride, uin
                            uint32_t q_pitch, float *d, uint32_t d_ld, uint32_t S, size_t pstride, uint32_t ileave) {
     const bool vec = ((uintptr_t)gu & 15) == 0 && gu_stride % 4 == 0 && pstride % 4 == 0 && F % 32 == 0 && ileave % 4 == 0 && ((uintptr_t)q & 3) == 0 &&
                      q_pitch % 4 == 0;
-    if (vec)
+    if (vec) {
         QB_CUDA(qb_launch_pdl(ctx->stream, swiglu_quant4_kernel, dim3((F + 1023) / 1024, M), dim3(256), (size_t)(0), gu, gu_stride, F, q, q_pitch, d, d_ld, S,
                               pstride, ileave));
-    else
-        QB_CUDA(qb_launch_pdl(ctx->stream, swiglu_quant_kernel, dim3((F / 32 + 7) / 8, M), dim3(256), (size_t)(0), gu, gu_stride, F, q, q_pitch, d, d_ld, S,
-                              pstride, ileave));
+        QB_LAUNCHED(ctx, "swiglu_quant4_kernel");
+        return QB_OK;
+    }
+    QB_CUDA(qb_launch_pdl(ctx->stream, swiglu_quant_kernel, dim3((F / 32 + 7) / 8, M), dim3(256), (size_t)(0), gu, gu_stride, F, q, q_pitch, d, d_ld, S, pstride,
+                          ileave));
     QB_LAUNCHED(ctx, "swiglu_quant_kernel");
     return QB_OK;
 }

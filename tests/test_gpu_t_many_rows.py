@@ -214,6 +214,31 @@ def test_merge_that_fills_the_gpu_equals_small_ones(qb, ctx, rows, pos, heads, k
         np.testing.assert_array_equal(whole[lo:lo + 16], run(lo, min(lo + 16, rows)))
 
 
+def test_launches_are_reported_under_their_own_names(qb, ctx):
+    """The launch trace (and the message of a failed launch) names the kernel that ran: many rows and few rows take different ones."""
+    L, x, w = qb.lib(), ctx.array(np.ones((600, 1024), np.float32)), ctx.array(np.ones(1024, np.float32))
+    y, q, d = ctx.empty((600, 1024), np.float32), ctx.empty((600, 1024), np.int8), ctx.empty((32, 600), np.float32)
+    gate_up = qb.Weight.synth(ctx, 1, 2, 2048, 1024)
+    cache, table = ctx.empty((600 * 2 * 256,), np.float16), ctx.array(np.arange(38, dtype=np.int32))
+    cache.zero()
+    qkv, out, pos = ctx.array(np.ones((600, 2 * 8 * 256 + 4 * 256), np.float32)), ctx.empty((600, 8 * 256), np.float32), ctx.array(np.zeros(1, np.int32))
+
+    def names(rows):
+        ctx.trace_enable(True)
+        for st in (L.qb_rms_norm(ctx.h, x.ptr, w.ptr, rows, 1024, 1024, C.c_float(1e-6), y.ptr),
+                   L.qb_q8_0_matmul_silu_mul_q8(ctx.h, gate_up.h, x.ptr, rows, 1024, q.ptr, d.ptr, 1),
+                   L.qb_attention_paged_gated(ctx.h, qkv.ptr, rows, 2 * 8 * 256 + 4 * 256, 8, 2, 256, pos.ptr, 1, table.ptr, 38, 16, cache.ptr, cache.ptr, rows, out.ptr)):
+            qb.binding.check(st)
+        seen = {n for n, _, _ in ctx.trace_summary()}
+        ctx.trace_enable(False)
+        return seen
+
+    many, few = names(600), names(8)
+    assert {"norm_quant_rows_kernel", "swiglu_quant4_kernel", "attn_merge4_kernel"} <= many and not {"norm_quant_kernel", "attn_merge_kernel"} & many
+    assert {"norm_quant_kernel", "attn_merge_kernel"} <= few and not {"norm_quant_rows_kernel", "attn_merge4_kernel"} & few
+    gate_up.free()
+
+
 def prompt_logits(qb, model, toks, max_ctx):
     b = qb.Batch(model, 1, max_ctx, 0)
     b.prefill(0, toks)
