@@ -664,7 +664,10 @@ int launch_ingest(qb_ctx *ctx, const DnArgs &a) {
     float *work = a.work;
     if (!work || need > a.work_floats) {
         void *p = nullptr;
-        QB_TRY(qb_ctx_scratch3(ctx, need * sizeof(float), &p));
+        if (qb_ctx_scratch3(ctx, need * sizeof(float), &p) != QB_OK) {       // no room on the device: the one-kernel form, the same bits
+            cudaGetLastError();
+            return launch_fused<HD, 4, 8, 1>(ctx, a);
+        }
         work = (float *)p;
     }
     float *qk = work, *vc = work + nqk, *gb = vc + nvc;

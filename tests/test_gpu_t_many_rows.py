@@ -78,6 +78,45 @@ def test_deltanet_checkpoints_of_many_rows_equal_single_rows(qb, ctx, nk, nv, hd
         assert np.array_equal(d_state.download()[:, 0], states[:, t]) and np.array_equal(d_conv.download()[:, 0], convs[:, t]), t
 
 
+def test_deltanet_prompt_rows_where_the_device_has_no_room_for_a_workspace(qb):
+    """qb_deltanet_rows without room for the three-launch form's workspace runs the one-kernel form: the same bits, no error."""
+    c = qb.Context(0)                                        # (its workspace does not exist yet)
+    nk, nv, hd, R = 16, 48, 128, 512                         # 21 MB of workspace
+    rng = np.random.default_rng(5)
+    Cq, stride = (2 * nk + nv) * hd, (2 * nk + 2 * nv) * hd + 2 * nv
+    proj = c.array(rng.standard_normal((R, stride), dtype=np.float32))
+    cw, sa, dt, nw = c.array(rng.uniform(-0.5, 0.5, (Cq, 4)).astype(np.float32)), c.array(-np.ones(nv, np.float32)), c.array(-np.ones(nv, np.float32)), c.array(np.ones(hd, np.float32))
+    state, conv, core, slot = c.empty((nv, hd, hd), np.float32), c.empty((Cq, 3), np.float32), c.empty((R, nv * hd), np.float32), c.array(np.zeros(1, np.int32))
+
+    def run(rows):
+        state.zero()
+        conv.zero()
+        c.trace_enable(True)
+        qb.binding.check(qb.lib().qb_deltanet_rows(c.h, proj.ptr, 1, rows, stride, cw.ptr, sa.ptr, dt.ptr, nw.ptr, nk, nv, hd, C.c_float(1e-6), state.ptr, conv.ptr,
+                                                   1, slot.ptr, 0, core.ptr))
+        ran = {n for n, _, _ in c.trace_summary()}
+        c.trace_enable(False)
+        return ran, core.download()[:rows], state.download(), conv.download()
+
+    run(15)                                                  # the scratch that every call needs
+    size, filler = c.mem_info()[0] - (6 << 20), None
+    while filler is None:
+        try:
+            filler = c.empty(size, np.uint8)
+        except qb.QbError:
+            size -= 4 << 20
+    try:
+        assert c.mem_info()[0] < 20 << 20
+        got = run(R)
+    finally:
+        filler.free()
+    want = run(R)
+    assert got[0] == {"dn_fused_kernel"} and "dn_scan_kernel" in want[0]
+    for a, b in zip(got[1:], want[1:]):
+        assert np.array_equal(a, b)
+    c.close()
+
+
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64, 65, 100])
 @pytest.mark.parametrize("N,K,stride", [(64, 32, 32), (130, 100, 101), (9600, 64, 68), (200, 2056, 2056)])
 def test_dense_product_in_32_bits(qb, ctx, M, N, K, stride):
