@@ -165,9 +165,8 @@ __global__ void __launch_bounds__(512, MINB) dn_fused_kernel(DnArgs a) {
         for (int t = 0; t < RB; ++t) {
             x[t] = 0.0f;
             if (has && (uint32_t)t < nrows) {
-                float acc = w[3] * cur[t];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) acc += w[k] * st[k];
+                float acc = fmaf(w[3], cur[t], __fmul_rn(w[0], st[0]));
+                acc = fmaf(w[2], st[2], fmaf(w[1], st[1], acc));
                 x[t] = __fdiv_rn(acc, 1.0f + expf(-acc));
                 st[0] = st[1]; st[1] = st[2]; st[2] = cur[t];
                 if (writes && a.write_all && rb0 + t < a.n_slots) {
@@ -228,7 +227,7 @@ __global__ void __launch_bounds__(512, MINB) dn_fused_kernel(DnArgs a) {
                 for (int cc = 0; cc < 4; ++cc) {
                     float kv = 0.0f;
 #pragma unroll
-                    for (int r = 0; r < RPL; ++r) kv += s[cc][r] * kr[r];
+                    for (int r = 0; r < RPL; ++r) kv = fmaf(s[cc][r], kr[r], kv);
                     kvp[cc] = kv;
                 }
                 const float kvt = sum4(kvp);
@@ -236,12 +235,12 @@ __global__ void __launch_bounds__(512, MINB) dn_fused_kernel(DnArgs a) {
 #pragma unroll
                 for (int cc = 0; cc < 4; ++cc) {
                     const float kv = __shfl_sync(0xffffffffu, kvt, 8 * (cc & 1) + 16 * (cc >> 1));
-                    const float delta = (xs[t][2 * HD + warp * CPW + cc] - g * kv) * beta;
+                    const float delta = __fmul_rn(fmaf(-g, kv, xs[t][2 * HD + warp * CPW + cc]), beta);
                     float at = 0.0f;
 #pragma unroll
                     for (int r = 0; r < RPL; ++r) {
-                        s[cc][r] = g * s[cc][r] + kr[r] * delta;
-                        at += s[cc][r] * qr[r];
+                        s[cc][r] = fmaf(g, s[cc][r], __fmul_rn(kr[r], delta));
+                        at = fmaf(s[cc][r], qr[r], at);
                     }
                     atp[cc] = at;
                     if (a.write_all && rb0 + t < a.n_slots) {
@@ -270,19 +269,19 @@ __global__ void __launch_bounds__(512, MINB) dn_fused_kernel(DnArgs a) {
                 for (int cc = 0; cc < 2; ++cc) {
                     float kv = 0.0f;
 #pragma unroll
-                    for (int r = 0; r < RPL; ++r) kv += s[cc][r] * kr[r];
+                    for (int r = 0; r < RPL; ++r) kv = fmaf(s[cc][r], kr[r], kv);
                     kvp[cc] = kv;
                 }
                 const float kvt = sum2(kvp[0], kvp[1]);
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {
                     const float kv = __shfl_sync(0xffffffffu, kvt, 16 * cc);
-                    const float delta = (xs[t][2 * HD + warp * CPW + cc] - g * kv) * beta;
+                    const float delta = __fmul_rn(fmaf(-g, kv, xs[t][2 * HD + warp * CPW + cc]), beta);
                     float at = 0.0f;
 #pragma unroll
                     for (int r = 0; r < RPL; ++r) {
-                        s[cc][r] = g * s[cc][r] + kr[r] * delta;
-                        at += s[cc][r] * qr[r];
+                        s[cc][r] = fmaf(g, s[cc][r], __fmul_rn(kr[r], delta));
+                        at = fmaf(s[cc][r], qr[r], at);
                     }
                     atp[cc] = at;
                     if (a.write_all && rb0 + t < a.n_slots) {
@@ -298,14 +297,14 @@ __global__ void __launch_bounds__(512, MINB) dn_fused_kernel(DnArgs a) {
             for (int cc = 0; cc < CPW; ++cc) {
                 float kv = 0.0f;
 #pragma unroll
-                for (int r = 0; r < RPL; ++r) kv += s[cc][r] * kr[r];
+                for (int r = 0; r < RPL; ++r) kv = fmaf(s[cc][r], kr[r], kv);
                 kv = warp_sum(kv);
-                const float delta = (xs[t][2 * HD + warp * CPW + cc] - g * kv) * beta;
+                const float delta = __fmul_rn(fmaf(-g, kv, xs[t][2 * HD + warp * CPW + cc]), beta);
                 float at = 0.0f;
 #pragma unroll
                 for (int r = 0; r < RPL; ++r) {
-                    s[cc][r] = g * s[cc][r] + kr[r] * delta;
-                    at += s[cc][r] * qr[r];
+                    s[cc][r] = fmaf(g, s[cc][r], __fmul_rn(kr[r], delta));
+                    at = fmaf(s[cc][r], qr[r], at);
                 }
                 at = warp_sum(at);
                 if (lane == 0) core_s[t][warp * CPW + cc] = at * oscale;
@@ -402,7 +401,8 @@ int launch_fused(qb_ctx *ctx, const DnArgs &a) {
 //                    exchange steps instead of five, the first shared by the columns of a thread; rows arrive by cp.async
 //   dn_gate_kernel   head-wide RMSNorm * gain * SiLU(z), quantisation, all rows at once
 // Every sum is formed from the same pairs in the same order as in dn_fused_kernel (a lane adds the partial sums of the four lanes
-// it stands for as the first two exchange steps would), so a row has the same bits in either form.
+// it stands for as the first two exchange steps would), and every product that enters a sum is a written fma, so a row has the same bits in
+// either form.
 constexpr uint32_t DN_PB = 8;                    // rows per block of the two parallel kernels
 
 // q and k are stored so that a lane of the scan reads its values with 16-byte loads: inside every 32 values, index 8j + m is at 4m + j.
@@ -448,9 +448,8 @@ __global__ void __launch_bounds__(HD) dn_prep_kernel(DnArgs a, float *__restrict
     float x[DN_PB];
 #pragma unroll
     for (int t = 0; t < (int)DN_PB; ++t) {
-        float acc = w[3] * cur[3 + t];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) acc += w[k] * cur[t + k];
+        float acc = fmaf(w[3], cur[3 + t], __fmul_rn(w[0], cur[t]));
+        acc = fmaf(w[2], cur[t + 2], fmaf(w[1], cur[t + 1], acc));
         x[t] = __fdiv_rn(acc, 1.0f + expf(-acc));
     }
     if (is_qk) {
@@ -584,7 +583,7 @@ __global__ void __launch_bounds__(32 * NW) dn_scan_kernel(DnArgs a, const float 
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
                 const float kv = __shfl_sync(0xffffffffu, kvt, CPT == 4 ? 4 * (c >> 1) + 2 * (c & 1) : 4 * c, 8);
-                const float delta = (row[2 * HD + lc + c] - g * kv) * beta;
+                const float delta = __fmul_rn(fmaf(-g, kv, row[2 * HD + lc + c]), beta);
                 const f32x2 d2 = pack2(delta, delta);
                 f32x2 lo = pack2(0.0f, 0.0f), hi = lo;
 #pragma unroll
