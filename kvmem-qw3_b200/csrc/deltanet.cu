@@ -394,7 +394,7 @@ int launch_fused(qb_ctx *ctx, const DnArgs &a) {
 
 // ---- prompt ingestion: three launches per layer ---------------------------------------------------------------
 // One CTA of dn_fused_kernel spends most of a row waiting: two five-step exchanges over 32 lanes, the barriers of the conv and
-// norm phases, one CTA per SM (595 us per 512 rows and layer at 48 heads of 128; these three 220, the scan 175).  Only the delta rule is
+// norm phases, one CTA per SM (550 us per 512 rows and layer at 48 heads of 128; these three 212, the scan 190 of them).  Only the delta rule is
 // sequential, so for many rows everything else leaves that chain:
 //   dn_prep_kernel   conv + SiLU, L2 norm, gates of all rows at once
 //   dn_scan_kernel   the delta rule; a column of the state is held by 8 lanes (16 of its 128 values each at head size 128): three
@@ -409,7 +409,8 @@ constexpr uint32_t DN_PB = 8;                    // rows per block of the two pa
 template <int HD>
 __global__ void __launch_bounds__(HD) dn_prep_kernel(DnArgs a, float *__restrict__ qk, float *__restrict__ vc, float *__restrict__ gb) {
     // No early start of the scan: its CTAs would be placed while this kernel's still fill most SMs, several of them on the SMs that
-    // are free first, and the scan's time is that of its fullest SM (500 us instead of 255 per 512 rows).
+    // are free first, and the scan's time is that of its fullest SM (its first form, scalar and with four columns a thread, took 500 us
+    // in the stream where it took 255 alone).
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float red[DN_PB][HD / 32];
     const uint32_t u = blockIdx.x, rb0 = blockIdx.y * DN_PB, seq = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -490,13 +491,12 @@ __global__ void __launch_bounds__(HD) dn_prep_kernel(DnArgs a, float *__restrict
     }
 }
 
-// grid (HD / COLS, nv, n_seqs): a CTA owns COLS = NW * 4 * CPT state columns of a head, a thread 1/8 of CPT columns.  The core
+// grid (HD / COLS, nv, n_seqs): a CTA owns COLS = 8 NW state columns of a head, a thread 1/8 of CPT = 2 columns.  The core
 // output takes the place of v in vc (a CTA has read a row's v before it writes that row).
-template <int HD, int CPT, int NW>
+template <int HD, int NW>
 __global__ void __launch_bounds__(32 * NW) dn_scan_kernel(DnArgs a, const float *__restrict__ qk, float *vc, const float *__restrict__ gb) {
     QB_PDL_ENTER();
-    constexpr int COLS = NW * 4 * CPT, NR = HD / 32, TR = 16, PITCH = 2 * HD + COLS + 4;
-    static_assert(CPT == 2 || CPT == 4, "columns per thread");
+    constexpr int CPT = 2, COLS = NW * 4 * CPT, NR = HD / 32, TR = 16, PITCH = 2 * HD + COLS + 4;
     __shared__ __align__(16) float buf[2][TR][PITCH];
     const uint32_t vh = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t m = lane & 7, lc = warp * 4 * CPT + (lane >> 3) * CPT, kh = vh % a.nk, R = a.rows_per_seq, vdim = a.nv * HD;
@@ -527,25 +527,13 @@ __global__ void __launch_bounds__(32 * NW) dn_scan_kernel(DnArgs a, const float 
 #pragma unroll
             for (int j = 0; j < 2; ++j) s[c][r][j] = pack2(st_in[(size_t)c * HD + r * 32 + 16 * j], st_in[(size_t)c * HD + r * 32 + 16 * j + 8]);
     const float oscale = rsqrtf((float)HD);
-    const bool hi4 = (m & 4) != 0, hi2 = (m & 2) != 0;
-    // Totals over a column's 8 lanes: the first step (CPT 4: the first two) halves the columns a lane carries.  The lane ends with the
-    // total of column 2 * hi4 + hi2 (CPT 4) or hi4 (CPT 2).
+    const bool hi4 = (m & 4) != 0;
+    // Totals over a column's 8 lanes: the first step halves the columns a lane carries, which ends with the total of column hi4.
     auto total = [&](const float (&v)[CPT]) -> float {
-        float k;
-        if constexpr (CPT == 4) {
-            float k0 = hi4 ? v[2] : v[0], k1 = hi4 ? v[3] : v[1];
-            const float s0 = hi4 ? v[0] : v[2], s1 = hi4 ? v[1] : v[3];
-            k0 += __shfl_xor_sync(0xffffffffu, s0, 4);
-            k1 += __shfl_xor_sync(0xffffffffu, s1, 4);
-            k = hi2 ? k1 : k0;
-            const float sd = hi2 ? k0 : k1;
-            k += __shfl_xor_sync(0xffffffffu, sd, 2);
-        } else {
-            k = hi4 ? v[1] : v[0];
-            const float sd = hi4 ? v[0] : v[1];
-            k += __shfl_xor_sync(0xffffffffu, sd, 4);
-            k += __shfl_xor_sync(0xffffffffu, k, 2);
-        }
+        float k = hi4 ? v[1] : v[0];
+        const float sd = hi4 ? v[0] : v[1];
+        k += __shfl_xor_sync(0xffffffffu, sd, 4);
+        k += __shfl_xor_sync(0xffffffffu, k, 2);
         return k + __shfl_xor_sync(0xffffffffu, k, 1);
     };
     for (uint32_t t0 = 0, bf = 0; t0 < R; t0 += TR, bf ^= 1) {
@@ -582,7 +570,7 @@ __global__ void __launch_bounds__(32 * NW) dn_scan_kernel(DnArgs a, const float 
             const float kvt = total(part);
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
-                const float kv = __shfl_sync(0xffffffffu, kvt, CPT == 4 ? 4 * (c >> 1) + 2 * (c & 1) : 4 * c, 8);
+                const float kv = __shfl_sync(0xffffffffu, kvt, 4 * c, 8);
                 const float delta = __fmul_rn(fmaf(-g, kv, row[2 * HD + lc + c]), beta);
                 const f32x2 d2 = pack2(delta, delta);
                 f32x2 lo = pack2(0.0f, 0.0f), hi = lo;
@@ -596,7 +584,7 @@ __global__ void __launch_bounds__(32 * NW) dn_scan_kernel(DnArgs a, const float 
                 part[c] = fold(lo, hi);
             }
             const float att = total(part);
-            if (CPT == 4 ? (m & 1) == 0 : (m & 3) == 0) v_src[(size_t)(t0 + t) * vdim + lc + (CPT == 4 ? m >> 1 : m >> 2)] = att * oscale;
+            if ((m & 3) == 0) v_src[(size_t)(t0 + t) * vdim + lc + (m >> 2)] = att * oscale;
         }
         __syncthreads();                                         // the buffer is free for the fetch of the next round
     }
@@ -656,9 +644,9 @@ __global__ void __launch_bounds__(HD) dn_gate_kernel(DnArgs a, const float *__re
 
 template <int HD>
 int launch_ingest(qb_ctx *ctx, const DnArgs &a) {
-    // 64 columns per CTA, two per thread.  Measured per 512 rows, all three launches: 2 columns x 8 warps 226 us, 2 x 4 252,
-    // 4 x 4 285, 4 x 2 292, 4 x 1 318.
-    constexpr int CPT = 2, NW = 8;
+    // 64 columns per CTA, two per thread: 96 CTAs of 8 warps at 48 heads.  Measured per 512 rows, all three launches, side by side: 2 columns
+    // x 8 warps 226 us, 2 x 4 252, 4 x 4 285, 4 x 2 292, 4 x 1 318 (212 for the first on its own, between events on a quiet stream).
+    constexpr int NW = 8, COLS = 8 * NW;
     const size_t rows = (size_t)a.n_seqs * a.rows_per_seq, nqk = rows * a.nk * 2 * HD, nvc = rows * a.nv * HD, need = nqk + nvc + rows * 2 * a.nv;
     float *work = a.work;
     if (!work || need > a.work_floats) {
@@ -673,7 +661,7 @@ int launch_ingest(qb_ctx *ctx, const DnArgs &a) {
     const uint32_t rblk = (a.rows_per_seq + DN_PB - 1) / DN_PB;
     QB_CUDA(qb_launch_pdl(ctx->stream, dn_prep_kernel<HD>, dim3(2 * a.nk + a.nv, rblk, a.n_seqs), dim3(HD), 0, a, qk, vc, gb));
     QB_LAUNCHED(ctx, "dn_prep_kernel");
-    QB_CUDA(qb_launch_pdl(ctx->stream, dn_scan_kernel<HD, CPT, NW>, dim3(HD / (NW * 4 * CPT), a.nv, a.n_seqs), dim3(32 * NW), 0, a, (const float *)qk, vc, (const float *)gb));
+    QB_CUDA(qb_launch_pdl(ctx->stream, dn_scan_kernel<HD, NW>, dim3(HD / COLS, a.nv, a.n_seqs), dim3(32 * NW), 0, a, (const float *)qk, vc, (const float *)gb));
     QB_LAUNCHED(ctx, "dn_scan_kernel");
     QB_CUDA(qb_launch_pdl(ctx->stream, dn_gate_kernel<HD>, dim3(a.nv, rblk, a.n_seqs), dim3(HD), 0, a, (const float *)vc));
     QB_LAUNCHED(ctx, "dn_gate_kernel");
