@@ -431,7 +431,8 @@ int qb_launch_sample_rows(qb_ctx *ctx, const float *logits, uint32_t rows, uint3
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    // the loops over a thread's elements are unrolled: vocabularies up to 32768 take the form with 4 of them
+    // The loops over a thread's elements are unrolled for the most it can have: 20, or 4 for vocabularies of up to 32768 (the widest that
+    // gives a thread no more; 1 / 128 rows of 32768 logits 107 / 975 us with 20, 69 / 624 with 4).
     const auto kernel = V <= (uint32_t)(CL * ST * 4) ? sample_rows_kernel<4> : sample_rows_kernel<EPT_MAX>;
     QB_CUDA(cudaLaunchKernelEx(&cfg, kernel, logits, V, stride, draft, u_acc, u_res, p, token, accepted, p_draft, pval,
                                pidx, nblk, K1));

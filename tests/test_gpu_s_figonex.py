@@ -249,8 +249,9 @@ def test_engine_chunks(make, monkeypatch):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-def test_long_prompt(make, dtype):
-    """More than one of the executor's 1024-token chunks: attention tiles of every fill, many blocks of the recurrences."""
+def test_long_prompt(make, monkeypatch, dtype):
+    """More than one pass of 1024 tokens: attention tiles of every fill, many blocks of the recurrences."""
+    monkeypatch.setenv("QW3B200_PREFILL_CHUNK", "1024")      # (the batch's own would hold the prompt in one)
     c = make(config([att(heads=8, kv=2, dim=64, rot=16, scale=0.5), lig(), mls()]))
     toks = c.tokens(1500)
     at = [0, 1, 127, 128, 500, 1022, 1023, 1024, 1025, 1151, 1152, 1498, 1499]

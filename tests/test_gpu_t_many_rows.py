@@ -120,8 +120,9 @@ def test_deltanet_prompt_rows_where_the_device_has_no_room_for_a_workspace(qb):
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64, 65, 100])
 @pytest.mark.parametrize("N,K,stride", [(64, 32, 32), (130, 100, 101), (9600, 64, 68), (200, 2056, 2056)])
 def test_dense_product_in_32_bits(qb, ctx, M, N, K, stride):
-    """Every tile of the fp32 product (rows and columns around its edges, odd strides) against 64 bits.  An output is four chains of K / 4
-    fused multiply-adds and two additions: at most (K / 4 + 2) roundings of half a unit in the last place of sum |x w|.
+    """Every tile of the fp32 product (rows and columns around its edges, odd strides) against 64 bits.  An output is four chains
+    of fused multiply-adds, one per 8 of every 32 k (up to 8 ceil(K / 32) of them), and two additions: at most that many and two roundings
+    of half a unit in the last place of sum |x w|.
     The same bits whatever the number of rows."""
     rng = np.random.default_rng(M + N + K)
     w = (rng.standard_normal((N, K)) * 0.05).astype(np.float32)
@@ -137,7 +138,7 @@ def test_dense_product_in_32_bits(qb, ctx, M, N, K, stride):
     got, first = y.download(), y1.download()
     L.qb_dense_weight_free(ctx.h, h)
     want = x[:, :K].astype(np.float64) @ w.T.astype(np.float64)
-    bound = (K / 4 + 2) * 2.0 ** -24 * (np.abs(x[:, :K]).astype(np.float64) @ np.abs(w.T).astype(np.float64))
+    bound = (8 * -(-K // 32) + 2) * 2.0 ** -24 * (np.abs(x[:, :K]).astype(np.float64) @ np.abs(w.T).astype(np.float64))
     assert (np.abs(got - want) <= bound).all()
     assert np.array_equal(got[:1], first)
 
@@ -253,6 +254,81 @@ def test_merge_that_fills_the_gpu_equals_small_ones(qb, ctx, rows, pos, heads, k
         np.testing.assert_array_equal(whole[lo:lo + 16], run(lo, min(lo + 16, rows)))
 
 
+@pytest.mark.parametrize("F,K", [(1024, 256), (3072, 1024), (18944, 256)])
+@pytest.mark.parametrize("M", [1, 5, 17, 130])
+def test_feed_forward_input_by_either_kernel(qb, ctx, M, F, K):
+    """One and several K segments: 16-byte pieces equal the scalar kernel, which an output that is not 4-byte aligned takes."""
+    L, w = qb.lib(), qb.Weight.synth(ctx, 12, 5, 2 * F, K, 0.02)
+    x = ctx.array(np.random.default_rng(M + F).standard_normal((M, K)).astype(np.float32))
+    ld = (M + 3) // 4 * 4
+
+    def run(shift):
+        q, d = ctx.empty((M * F + 16,), np.int8), ctx.empty((F // 32, ld), np.float32)
+        qb.binding.check(L.qb_q8_0_matmul_silu_mul_q8(ctx.h, w.h, x.ptr, M, K, C.c_void_p(q.ptr.value + shift), d.ptr, 1))
+        return q.download()[shift:shift + M * F], d.download()[:, :M]
+
+    (q, d), (qs, ds) = run(0), run(1)
+    assert np.any(q) and np.array_equal(q, qs) and np.array_equal(d, ds)
+    w.free()
+
+
+@pytest.mark.parametrize("M", [65, 130])
+def test_sharded_feed_forward_of_many_rows(qb, orc, ctx, M):
+    """Two ranks in one process, every push before any reduce: gate and up in halves (not interleaved), the 128-row tile pushing its sums to
+    both (one K segment of the down shard).  The receive areas hold every rank's product, the result their sum in rank order."""
+    H, F, n_out, world = 256, 512, 19072, 2
+    rng = np.random.default_rng(M)
+    f = F // world
+    gate, up = (orc.quantize_q8_0(rng.normal(0, 0.05, (F, H)).astype(np.float32)) for _ in range(2))
+    down = orc.quantize_q8_0(rng.normal(0, 0.05, (n_out, F)).astype(np.float32))
+    assert orc.ksplit_policy(n_out, f) == 1 and orc.ksplit_policy(2 * f, H) > 1
+    x = rng.normal(0, 1, (M, H)).astype(np.float32)
+    shards = [qb.tp.shard_blocks(gate, up, down, F, H, n_out, world, r) for r in range(world)]
+    wts = [(qb.Weight.from_blocks(ctx, gu, 2 * f, H), qb.Weight.from_blocks(ctx, dn, n_out, f)) for gu, dn in shards]
+    groups, areas = qb.tp.local_groups(ctx, world, M, H, f, n_out)
+    xd, ys = ctx.array(x), [ctx.empty((M, n_out), np.float32) for _ in range(world)]
+    for r in range(world):
+        groups[r].push(wts[r][0], wts[r][1], xd, M)
+    for r in range(world):
+        groups[r].reduce(M, ys[r])
+    ctx.sync()
+    got = [y.download() for y in ys]
+    want, parts = None, areas[0].download()[256:].view(np.float32)[:world * M * n_out].reshape(world, M, n_out)
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], parts[0] + parts[1])
+    for r in range(world):
+        q, d = orc.quantize_act(x)
+        y = orc.gemm_engine(shards[r][0], 2 * f, H, q, d)
+        h = (y[:, :f] / (np.float32(1) + np.exp(-y[:, :f], dtype=np.float32)) * y[:, f:]).astype(np.float32)
+        hq, hd = orc.quantize_act(h)
+        mine = orc.gemm_engine(shards[r][1], n_out, f, hq, hd)
+        # the device's expf may flip an int8 of the hidden row, no more
+        assert np.abs(parts[r] - mine).max() < 5e-3 * np.abs(mine).max()
+        want = mine if want is None else want + mine
+    assert np.abs(got[0] - want).max() < 5e-3 * np.abs(want).max()
+    for g in groups:
+        g.close()
+    for pair in wts:
+        pair[0].free(); pair[1].free()
+
+
+@pytest.mark.parametrize("V", [4096, 8191, 8193, 32767, 32768, 32769])
+@pytest.mark.parametrize("temp,top_p,top_k,min_p", [(0.7, 0.9, 0, 0.0), (0.8, 0.95, 20, 0.0), (1e6, 1.0, 0, 0.0)])
+def test_sampling_around_its_unrolled_forms(qb, orc, ctx, V, temp, top_p, top_k, min_p):
+    """Vocabularies of up to 32768 take the form unrolled for four logits a thread: either side of that edge and of the thread counts."""
+    rng = np.random.default_rng(V)
+    x = (rng.standard_normal((6, V)) * 3).astype(np.float32)
+    x[1, V - 1] = x[1].max() + 1
+    draft = np.array([-1, V - 1, -1, int(x[3].argmax()), 0, -1], np.int32)
+    ua, ur = rng.random(6), rng.random(6)
+    ur[0], ur[2] = 0.0, 1.0 - 1e-12
+    want = orc.sample_rows(x, draft, ua, ur, temp, top_p, top_k, min_p)
+    tok, acc, pd = ctx.empty((6,), np.int32), ctx.empty((6,), np.int32), ctx.empty((6,), np.float32)
+    qb.binding.check(qb.lib().qb_sample_rows(ctx.h, ctx.array(x).ptr, 6, V, V, ctx.array(draft).ptr, ctx.array(ua).ptr, ctx.array(ur).ptr, temp, top_p, top_k,
+                                             min_p, tok.ptr, acc.ptr, pd.ptr))
+    assert np.allclose(pd.download(), want[2], rtol=2e-5, atol=1e-9)
+    assert np.array_equal(acc.download(), want[1]) and np.array_equal(tok.download(), want[0])
+
+
 def test_launches_are_reported_under_their_own_names(qb, ctx):
     """The launch trace (and the message of a failed launch) names the kernel that ran: many rows and few rows take different ones."""
     L, x, w = qb.lib(), ctx.array(np.ones((600, 1024), np.float32)), ctx.array(np.ones(1024, np.float32))
@@ -335,4 +411,79 @@ def test_hybrid_pass_keeps_its_memory_bounded_and_shrinks_where_there_is_none(qb
     finally:
         filler.free()
     assert rows in (512, 1024) and np.array_equal(got, want)
+    m.close()
+
+
+def test_hybrid_rows_have_the_same_bits_in_every_pass(qb, ctx, monkeypatch):
+    """Passes of 48, 512, 1024 and 2048 rows (few and many CTAs of the norms and merges, split sums, both forms of the DeltaNet rows, the
+    quantised outputs that the products read): logits along a prompt and of the steps behind it, bit for bit."""
+    m = qb.Model(ctx, qb.configs.qwen35_bench(1024, 2048, 4, vocab=1024), 5)
+    toks = (np.arange(2100) * 7919 % 1021).astype(np.int32)
+    at = [0, 1, 47, 48, 255, 511, 512, 800, 1023, 1024, 1500, 2047, 2048, 2098]
+    runs = []
+    for rows in ("48", "512", "1024", None):
+        if rows:
+            monkeypatch.setenv("QW3B200_PREFILL_CHUNK", rows)
+        else:
+            monkeypatch.delenv("QW3B200_PREFILL_CHUNK")
+        b = qb.Batch(m, 1, 2200, 0)
+        assert b.max_rows == int(rows or 2048)
+        lg = [b.score(0, toks[:-1], at)]
+        b.prefill(0, toks[-1:])
+        lg.append(b.last_logits(1))
+        for _ in range(3):
+            b.greedy_step()
+            lg.append(b.last_logits(1))
+        runs.append(np.concatenate(lg))
+        b.close()
+    assert np.isfinite(runs[0]).all() and runs[0].std() > 0
+    for r in runs[1:]:
+        assert np.array_equal(runs[0], r)
+    m.close()
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("family", ["kezilix", "figonex"])
+def test_layered_rows_in_passes_of_either_size(qb, ctx, monkeypatch, family, dtype):
+    """Passes of 1024 and of 2048 rows, none with a short end (2600 tokens): the same bits."""
+    make = qb.configs.kezilix_bench if family == "kezilix" else qb.configs.figonex_bench
+    m = qb.Model.layered_synth(ctx, make(512, 1024, 4, vocab=512), 3, dtype)
+    toks = (np.arange(2600) * 7919 % 509).astype(np.int32)
+    want, rows = prompt_logits(qb, m, toks, 2700)
+    monkeypatch.setenv("QW3B200_PREFILL_CHUNK", "1024")
+    got, less = prompt_logits(qb, m, toks, 2700)
+    assert (rows, less) == (2048, 1024) and np.isfinite(want).all() and np.array_equal(want, got)
+    m.close()
+
+
+@pytest.mark.parametrize("k", [0, 2])
+def test_restore_of_many_state_buffers(qb, ctx, k):
+    """A hybrid batch with 130 state buffers (two launches of the copies), states that are no multiple of a copy's piece, sizes with a tail of
+    single words: the steps after a restore repeat the steps after the snapshot, bit for bit, from either parity of the conv windows."""
+    cfg = qb.configs.tiny()
+    cfg.n_layers, cfg.ssm_num_v_heads = 56, 6
+    m = qb.Model(ctx, cfg, 9)
+    b = qb.Batch(m, 3, 300, k)
+    for i, n in enumerate((37, 5, 61)):
+        b.prefill(i, (np.arange(n) * 7919 % 4093).astype(np.int32))
+    b.mtp_step() if k else b.greedy_step()
+    snap = b.snapshot()
+
+    def steps(n):
+        out = []
+        for _ in range(n):
+            b.mtp_step() if k else b.greedy_step()
+            out.append((b.read_output(), b.last_logits(3 * (k + 1)).copy(), [b.position(i) for i in range(3)]))
+        return out
+
+    first = steps(5)
+    for n in (5, 4, 1):
+        before = ctx.launches
+        b.restore(snap)
+        assert ctx.launches - before == 2
+        again = steps(n)
+        for x, y in zip(first, again):
+            assert x[0] == y[0] and x[2] == y[2] and np.array_equal(x[1], y[1])
+    b.free_snapshot(snap)
+    b.close()
     m.close()
