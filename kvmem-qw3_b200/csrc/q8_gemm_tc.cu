@@ -55,7 +55,8 @@ struct TcCfg {
     static constexpr int CTAS_PER_SM = MT == 16 ? 2 : 1;
     // Second launch bound.  Left unspecified, the compiler keeps several variants at 64 registers with spills inside
     // the drain loop (it assumes more resident CTAs than the shared memory allows); told the real residency it uses
-    // 94-168 registers and no spills.  The 32-column variant measured faster with the default, so it keeps it (0).
+    // 94-168 registers, with 12 bytes of spill stores left in the 128-row variant and 106 in the 16-column one.  The 32-column
+    // variant measured faster with the default, so it keeps it (0).
     static constexpr int MIN_CTAS = MT == 32 ? 0 : CTAS_PER_SM;
     static constexpr int NSLOT = 512 / CTAS_PER_SM / (KPS * MT);
     static constexpr int TMEM_COLS = NSLOT * KPS * MT;
