@@ -677,8 +677,10 @@ int qb_launch_deltanet(qb_ctx *ctx, const DnArgs &a) {
     QB_REQUIRE(a.conv_out && a.conv_out != a.conv, "deltanet: the new conv state needs a buffer of its own");
     // one request: 32 state columns per CTA (more CTAs, shortest critical path); several: 64 per CTA (the per-CTA
     // work that does not depend on the column count — the head's q/k conv, the barriers — is paid half as often)
-    // 16 rows or more per sequence: the three-launch form where only the last state is kept (prompt ingestion; below 16 rows its two more
-    // launches cost what the shorter rows give), 64 columns per CTA and 8-row blocks where every row leaves a checkpoint
+    // 16 rows or more per sequence: the three-launch form where only the last state is kept (prompt ingestion), 64 columns per CTA and 8-row
+    // blocks where every row leaves a checkpoint.  One kernel / three launches, us, one sequence of 48 heads of 128: 2 rows 11.2 / 17.9, 4 rows
+    // 12.5 / 18.0, 8 rows 18.5 / 14.5, 15 rows 29.5 / 16.6, 16 rows (8-row blocks) 22.8 / 16.6; 32 sequences, 4 rows 111 / 76.  So the line could
+    // lie at 6 rows for calls without checkpoints; those are prompts and ends of prompts that short, and they keep the steps' kernel.
     const bool wide = a.n_seqs > 2, many = a.rows_per_seq >= 16, ingest = many && !a.write_all;
     if (a.hd == 128) return ingest ? launch_ingest<128>(ctx, a) : many ? launch_fused<128, 4, 8, 1>(ctx, a) : wide ? launch_fused<128, 4, 4, 2>(ctx, a) : launch_fused<128, 2, 4, 2>(ctx, a);
     if (a.hd == 64) return ingest ? launch_ingest<64>(ctx, a) : many ? launch_fused<64, 4, 8, 1>(ctx, a) : wide ? launch_fused<64, 4, 4, 2>(ctx, a) : launch_fused<64, 2, 4, 2>(ctx, a);

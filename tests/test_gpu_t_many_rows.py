@@ -178,6 +178,32 @@ def test_norm_and_quantiser_around_a_second_wave(qb, ctx, waves):
     test_norm_and_quantiser_of_many_rows_equal_few_rows(qb, ctx, int(waves[0] * ctx.sm_count) + waves[1], 1056)
 
 
+@pytest.mark.parametrize("M", [256, 300, 512])
+def test_norm_of_rows_that_are_not_aligned(qb, ctx, M):
+    """Rows that start off a 16-byte boundary, or whose stride is no multiple of four floats, are read word by word: the same bits as aligned
+    rows, in either form."""
+    rng, n = np.random.default_rng(M), 1056
+    x = rng.standard_normal((M, n)).astype(np.float32)
+    flat, wide = np.zeros(M * n + 1, np.float32), np.zeros((M, n + 1), np.float32)
+    flat[1:], wide[:, :n] = x.ravel(), x
+    xd, fd, wd, w, L = ctx.array(x), ctx.array(flat), ctx.array(wide), ctx.array(rng.uniform(0.5, 1.5, n).astype(np.float32)), qb.lib()
+
+    def norm(p):
+        out = ctx.empty((M, n), np.float32)
+        qb.binding.check(L.qb_rms_norm(ctx.h, p, w.ptr, M, n, n, C.c_float(1e-6), out.ptr))
+        return out.download()
+
+    def quant(p, stride):
+        q, d = ctx.empty((M, n), np.int8), ctx.empty((n // 32, (M + 3) // 4 * 4), np.float32)
+        qb.binding.check(L.qb_quantize_act(ctx.h, p, M, n, stride, q.ptr, d.ptr))
+        return q.download(), d.download()[:, :M]
+
+    assert np.array_equal(norm(xd.ptr), norm(C.c_void_p(fd.ptr.value + 4)))
+    for got in (quant(C.c_void_p(fd.ptr.value + 4), n), quant(wd.ptr, n + 1)):
+        for a, b in zip(quant(xd.ptr, n), got):
+            assert np.any(a) and np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("M", [16, 17, 65, 130])
 def test_feed_forward_input_of_many_rows_equals_one_launch_form(qb, orc, ctx, M):
     """silu(gate) * up quantised by the vectorised kernel (any rows) == the GEMM's own epilogue (up to 16 rows at a time)."""
