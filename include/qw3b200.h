@@ -133,8 +133,11 @@ int qb_q8_block_dots(qb_ctx *ctx, const qb_weight *w, const int8_t *q_dev, uint3
  * y[m][n] = sum_kb d_w[n][kb] * d_x[m][kb] * int32dot, fp32 in / fp32 out.
  *   order = 0: engine order (K segments of qb_ksplit_policy or `ksplit` if non-zero; sequential
  *              fma per 32-block inside a segment as in src/mmq_q8.cu:1738-1748; segments summed ascending)
- *   impl  = 0: automatic, 1: CUDA-core dp4a streaming kernel, 2: tcgen05 INT8 tensor-core kernel.
- * Both implementations produce identical bits. */
+ *   impl  = 0: automatic, 1: CUDA-core dp4a streaming kernel, 2: tensor-core kernels (tcgen05): INT8 operands, or from 256
+ *              rows on fp16 operands where that is faster.
+ * All of them produce identical bits.  The work area (int8 activations, scales, K-segment partial sums) belongs to the context and
+ * grows to the largest call's; for the fp16 operands it grows by 2 bytes per activation more, up to 128 MiB and where
+ * the device has room (the INT8 kernel runs otherwise). */
 int qb_q8_0_matmul(qb_ctx *ctx, const qb_weight *w, const float *x_dev, uint32_t M, uint32_t x_stride,
                    float *y_dev, uint32_t y_stride, uint32_t ksplit, int impl);
 /* The same product as qb_q8_0_matmul (identical bits) for callers that must not allocate device memory:
@@ -147,7 +150,8 @@ int qb_q8_0_matmul(qb_ctx *ctx, const qb_weight *w, const float *x_dev, uint32_t
 int qb_q8_0_matmul_noalloc(qb_ctx *ctx, const qb_weight *w, const float *x_dev, uint32_t M, uint32_t x_stride,
                            float *y_dev, uint32_t y_stride, uint32_t ksplit);
 /* Same product from already-quantised activations, leaving the per-segment partial sums:
- * part_dev = float [ksplit][M][N]. */
+ * part_dev = float [ksplit][M][N].  Works in these buffers alone: it allocates nothing, waits for nothing and can be captured
+ * (its tensor-core form is the INT8 kernel at every row count). */
 int qb_q8_gemm_partials(qb_ctx *ctx, const qb_weight *w, const int8_t *q_dev, const float *d_dev, uint32_t M,
                         float *part_dev, uint32_t ksplit, int impl);
 

@@ -55,7 +55,6 @@ extern "C" void qb_destroy(qb_ctx *ctx) {
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->scratch2) cudaFree(ctx->scratch2);
     if (ctx->scratch3) cudaFree(ctx->scratch3);
-    if (ctx->scratch4) cudaFree(ctx->scratch4);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -92,7 +91,35 @@ static int grow(qb_ctx *ctx, void *&buf, size_t &have, size_t bytes, void **out)
 int qb_ctx_scratch(qb_ctx *ctx, size_t bytes, void **out) { return grow(ctx, ctx->scratch, ctx->scratch_bytes, bytes, out); }
 int qb_ctx_scratch2(qb_ctx *ctx, size_t bytes, void **out) { return grow(ctx, ctx->scratch2, ctx->scratch2_bytes, bytes, out); }
 int qb_ctx_scratch3(qb_ctx *ctx, size_t bytes, void **out) { return grow(ctx, ctx->scratch3, ctx->scratch3_bytes, bytes, out); }
-int qb_ctx_scratch4(qb_ctx *ctx, size_t bytes, void **out) { return grow(ctx, ctx->scratch4, ctx->scratch4_bytes, bytes, out); }
+
+// The same as qb_ctx_scratch, for a call that is faster with `extra` more bytes behind its `bytes` and correct without: *has_extra says whether they are
+// there.  The wider buffer is had before the old one goes, so a device without room costs nothing but the extra bytes: one failed allocation, and
+// no further one until a smaller size is asked for or the device has more free memory than at the failure.  Never grown for the extra
+// alone while the stream is being captured (an allocation would end the capture).
+int qb_ctx_scratch_extra(qb_ctx *ctx, size_t bytes, size_t extra, void **out, bool *has_extra) {
+    const size_t all = bytes + extra;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (extra && all > ctx->scratch_bytes && cudaStreamIsCapturing(ctx->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+        size_t free = 0, total = 0;
+        const bool again = !ctx->scratch_denied || all < ctx->scratch_denied || (cudaMemGetInfo(&free, &total) == cudaSuccess && free > ctx->scratch_denied_free);
+        void *p = nullptr;
+        size_t want = all + (all >> 2) + (1u << 20);
+        if (again && cudaMalloc(&p, want) != cudaSuccess && cudaMalloc(&p, want = all) != cudaSuccess) p = nullptr;
+        cudaGetLastError();
+        if (p) {
+            ctx->scratch_denied = 0;
+            QB_CUDA(cudaStreamSynchronize(ctx->stream));
+            if (ctx->scratch) QB_CUDA(cudaFree(ctx->scratch));
+            ctx->scratch = p;
+            ctx->scratch_bytes = want;
+        } else if (again) {
+            ctx->scratch_denied = all;
+            if (cudaMemGetInfo(&ctx->scratch_denied_free, &total) != cudaSuccess) ctx->scratch_denied_free = SIZE_MAX;
+        }
+    }
+    *has_extra = extra && all <= ctx->scratch_bytes;
+    return qb_ctx_scratch(ctx, bytes, out);
+}
 
 extern "C" int qb_mem_info(qb_ctx *ctx, size_t *free_bytes, size_t *total_bytes) {
     QB_REQUIRE(ctx, "qb_mem_info: null context");

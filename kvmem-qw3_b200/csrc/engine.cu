@@ -448,6 +448,7 @@ static int qwen35_batch_alloc(qb_ctx *ctx, qb_batch *b, size_t slots) {
     {
         size_t ml = 0;
         const size_t acc = qb_attention_scratch_floats(rows, c.n_heads, c.head_dim, max_ctx + draft_k + 1, &ml, b->attn_split);
+        b->att_acc_floats = acc;
         QB_CUDA(cudaMalloc(&b->att_acc, acc * sizeof(float)));
         QB_CUDA(cudaMalloc(&b->att_ml, ml * sizeof(float)));
     }
@@ -558,14 +559,7 @@ static int batch_create(qb_ctx *ctx, qb_model *m, uint32_t n_seqs, uint32_t max_
         if (chunk == 0) chunk = m->arch->pass_rows(b);
         b->chunk = chunk;
         const int st = batch_fill(ctx, b, page_order, pool_pages);
-        if (st == QB_OK) {
-            // the context's fp16 activations of the many-row products, before the first prompt; without room those products take their int8 form
-            const uint32_t cols = std::max({b->xq_h.K, b->xq_attn.K, b->xq_dn.K, b->xq_ffn.K, b->xq_cat.K});
-            void *work = nullptr;
-            if (cols && b->rows_cap >= 256 && qb_ctx_scratch4(ctx, (size_t)b->rows_cap * cols * 2, &work) != QB_OK) cudaGetLastError();
-            *out = b;
-            return QB_OK;
-        }
+        if (st == QB_OK) { *out = b; return QB_OK; }
         const bool memory = cudaGetLastError() == cudaErrorMemoryAllocation;
         qb_batch_destroy(ctx, b);
         // where the device has no room for the wide pass, the narrower ones, down to the family's own, give the same bits
@@ -808,12 +802,19 @@ __global__ void advance_kernel(int32_t *pos, int32_t *sel, uint32_t s, int32_t a
 // forward passes
 // ================================================================================================
 
+// Work area of a product that writes to dst: b->act, which holds something only from a product into it (gate/up, the K/V rows of a kv_only block) to that
+// product's consumer and during the recurrence's launches; for those products the attention partials, which live from an attention
+// launch to its merge.  Both are wider than the 2 bytes a column that a product can use (act: 8 per feed-forward or attention column).
+static QbGemmWork gemm_work(const qb_batch *b, const float *dst) {
+    return dst == b->act ? QbGemmWork{b->att_acc, b->att_acc_floats * sizeof(float)} : QbGemmWork{b->act, b->act_floats * sizeof(float)};
+}
+
 // y[rows][N] = W x, written to dst (row stride N).
 static int gemm_to(qb_ctx *ctx, qb_batch *b, const qb_weight *w, const QBuf &x, uint32_t rows, float *dst, uint32_t S_override = 0) {
     const uint32_t S = S_override ? S_override : qb_ksplit(w->rows, w->cols);
-    if (S == 1) return qb_launch_gemm(ctx, w, x.q, x.d, rows, dst, 1, b->gemm_impl);
+    if (S == 1) return qb_launch_gemm(ctx, w, x.q, x.d, rows, dst, 1, b->gemm_impl, gemm_work(b, dst));
     QB_REQUIRE((size_t)S * rows * w->rows <= b->parts_floats, "split scratch too small");
-    QB_TRY(qb_launch_gemm(ctx, w, x.q, x.d, rows, b->parts, S, b->gemm_impl));
+    QB_TRY(qb_launch_gemm(ctx, w, x.q, x.d, rows, b->parts, S, b->gemm_impl, gemm_work(b, b->parts)));
     return qb_launch_reduce_parts(ctx, b->parts, S, rows, w->rows, dst, w->rows);
 }
 
@@ -823,7 +824,7 @@ static int gemm_parts(qb_ctx *ctx, qb_batch *b, const qb_weight *w, const QBuf &
     QB_REQUIRE((size_t)S * rows * w->rows <= b->parts_floats || S == 1, "split scratch too small");
     QB_REQUIRE((size_t)rows * w->rows <= b->parts_floats, "split scratch too small");
     *S_out = S;
-    return qb_launch_gemm(ctx, w, x.q, x.d, rows, b->parts, S, b->gemm_impl);
+    return qb_launch_gemm(ctx, w, x.q, x.d, rows, b->parts, S, b->gemm_impl, gemm_work(b, b->parts));
 }
 
 // h += parts ; xq = quant(rmsnorm(h) * w)
@@ -894,7 +895,7 @@ static int ffn_block(qb_ctx *ctx, qb_batch *b, const LayerW &L, float *h, uint32
         return residual_norm_quant(ctx, b, h, rows, 1, next_norm_w, b->xq_h, 0, true, b->tp_y);
     }
     QB_TRY(qb_ffn_gate_up_swiglu(ctx, L.w_gate_up, b->xq_h.q, b->xq_h.d, rows, b->act, b->parts, b->parts_floats, b->xq_ffn.q, b->xq_ffn.K,
-                                 b->xq_ffn.d, qb_act_ld(rows), b->gemm_impl, 0));
+                                 b->xq_ffn.d, qb_act_ld(rows), b->gemm_impl, 0, gemm_work(b, b->act)));
     uint32_t S = 1;
     QB_TRY(gemm_parts(ctx, b, L.w_down, b->xq_ffn, rows, &S));
     return residual_norm_quant(ctx, b, h, rows, S, next_norm_w, b->xq_h);

@@ -117,7 +117,7 @@ struct qb_batch {
     // activations
     float *hid = nullptr;                  // [rows_cap + n_seqs][H]; rows rows_cap+s hold prev hidden of seq s
     float *mtp_h = nullptr, *embd = nullptr, *act = nullptr, *parts = nullptr;
-    size_t act_floats = 0;
+    size_t act_floats = 0, att_acc_floats = 0;
     float *logits = nullptr, *am_val = nullptr, *att_acc = nullptr, *att_ml = nullptr;
     int32_t *am_idx = nullptr;
     QBuf xq_h, xq_attn, xq_dn, xq_ffn, xq_cat;

@@ -93,15 +93,18 @@ extern "C" int qb_q8_0_matmul_silu_mul_q8(qb_ctx *ctx, const qb_weight *gate_up,
     QB_REQUIRE(gate_up->rows % 128 == 0 && gate_up->cols % 128 == 0, "qb_q8_0_matmul_silu_mul_q8: weight must be whole 128 x 128 tiles");
     const uint32_t K = gate_up->cols, N = gate_up->rows, F = N / 2, ld = qb_act_ld(M), S = qb_ksplit(N, K);
     const size_t q_bytes = ((size_t)M * K + 255) & ~(size_t)255, d_bytes = ((size_t)(K / 32) * ld * 4 + 255) & ~(size_t)255;
-    const size_t act_floats = (size_t)S * M * N;
+    const size_t act_floats = (size_t)S * M * N, w_bytes = qb_gemm_work_bytes(ctx, gate_up, M, S, 0);      // (N is a multiple of 128: act ends on a 16-byte boundary)
     void *scr = nullptr;
-    QB_TRY(qb_ctx_scratch(ctx, q_bytes + d_bytes + act_floats * sizeof(float), &scr));
+    bool extra = false;
+    QB_TRY(qb_ctx_scratch_extra(ctx, q_bytes + d_bytes + act_floats * sizeof(float), w_bytes, &scr, &extra));
     int8_t *xq = (int8_t *)scr;
     float *xd = (float *)((uint8_t *)scr + q_bytes), *act = (float *)((uint8_t *)scr + q_bytes + d_bytes);
+    QbGemmWork work;
+    if (extra) { work.p = act + act_floats; work.bytes = w_bytes; }
     NormQuantArgs a;
     a.x = x_dev; a.x_stride = x_stride; a.n = K; a.M = M; a.q = xq; a.q_pitch = K; a.d = xd; a.d_ld = ld;
     QB_TRY(qb_launch_norm_quant(ctx, a));
-    return qb_ffn_gate_up_swiglu(ctx, gate_up, xq, xd, M, act, act, act_floats, hq_dev, F, hd_dev, ld, 0, mode);
+    return qb_ffn_gate_up_swiglu(ctx, gate_up, xq, xd, M, act, act, act_floats, hq_dev, F, hd_dev, ld, 0, mode, work);
 }
 
 namespace {

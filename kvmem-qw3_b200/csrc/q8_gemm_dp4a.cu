@@ -178,7 +178,7 @@ uint32_t qb_ksplit(uint32_t N, uint32_t K) {
 extern "C" uint32_t qb_ksplit_policy(uint32_t N, uint32_t K) { return qb_ksplit(N, K); }
 
 int qb_ffn_gate_up_swiglu(qb_ctx *ctx, const qb_weight *w, const int8_t *xq, const float *xd, uint32_t M, float *act, float *parts,
-                          size_t parts_floats, int8_t *hq, uint32_t hq_pitch, float *hd, uint32_t hd_ld, int gemm_impl, int mode) {
+                          size_t parts_floats, int8_t *hq, uint32_t hq_pitch, float *hd, uint32_t hd_ld, int gemm_impl, int mode, const QbGemmWork &work) {
     const uint32_t F = w->rows / 2, S = qb_ksplit(w->rows, w->cols);
     const bool can_fuse = M <= 16 && S == 1 && w->rows % 128 == 0 && w->cols / 128 > 8 && qb_gemm_tc_supported(w, M) && gemm_impl != 1;
     QB_REQUIRE(mode != 2 || can_fuse, "gate/up + SwiGLU in one launch needs M <= 16, one K segment and K > 1024");
@@ -193,11 +193,11 @@ int qb_ffn_gate_up_swiglu(qb_ctx *ctx, const qb_weight *w, const int8_t *xq, con
         return st;
     }
     if (S == 1) {
-        QB_TRY(qb_launch_gemm(ctx, w, xq, xd, M, act, 1, gemm_impl));
+        QB_TRY(qb_launch_gemm(ctx, w, xq, xd, M, act, 1, gemm_impl, work));
         return qb_launch_swiglu_quant(ctx, act, w->rows, M, F, hq, hq_pitch, hd, hd_ld, 1, 0, 64);
     }
     QB_REQUIRE((size_t)S * M * w->rows <= parts_floats, "split scratch too small");
-    QB_TRY(qb_launch_gemm(ctx, w, xq, xd, M, parts, S, gemm_impl));
+    QB_TRY(qb_launch_gemm(ctx, w, xq, xd, M, parts, S, gemm_impl, work));
     return qb_launch_swiglu_quant(ctx, parts, w->rows, M, F, hq, hq_pitch, hd, hd_ld, S, (size_t)M * w->rows, 64);
 }
 
@@ -210,7 +210,7 @@ int qb_launch_gemm_dp4a(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const 
 }
 
 static int gemm_dispatch(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const float *d, uint32_t M, float *part,
-                         uint32_t S, int impl);
+                         uint32_t S, int impl, const QbGemmWork &work);
 
 // Algorithmic bytes of one launch: the Q8_0 weight once (34 B per 32 weights), the quantised
 // activations (int8 + one fp32 scale per 32) and the fp32 partial sums written.
@@ -238,10 +238,10 @@ int qb_prof_end(qb_ctx *ctx, double bytes) {
 }
 
 int qb_launch_gemm(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const float *d, uint32_t M, float *part,
-                   uint32_t S, int impl) {
-    if (!ctx->prof_on) return gemm_dispatch(ctx, w, q, d, M, part, S, impl);
+                   uint32_t S, int impl, const QbGemmWork &work) {
+    if (!ctx->prof_on) return gemm_dispatch(ctx, w, q, d, M, part, S, impl, work);
     QB_TRY(qb_prof_begin(ctx));
-    const int st = gemm_dispatch(ctx, w, q, d, M, part, S, impl);
+    const int st = gemm_dispatch(ctx, w, q, d, M, part, S, impl, work);
     QB_TRY(qb_prof_end(ctx, gemm_bytes(w, M, S)));
     return st;
 }
@@ -266,13 +266,9 @@ extern "C" int qb_prof_summary(qb_ctx *ctx, double *total_ms, double *total_byte
     return QB_OK;
 }
 
-static int gemm_dispatch(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const float *d, uint32_t M, float *part,
-                         uint32_t S, int impl) {
-    if (impl == 2) {
-        if (!qb_gemm_tc_supported(w, M))
-            return qb_fail(QB_ERR_UNSUPPORTED, "tensor-core GEMM does not support this shape");
-        return qb_launch_gemm_tc(ctx, w, q, d, M, part, S);
-    }
+// Whether a product runs on the tensor cores.
+static bool takes_tc(const qb_weight *w, uint32_t M, int impl) {
+    if (impl == 2) return true;
     // automatic choice (measured): the tensor-core kernel everywhere except the matvec over a very tall weight
     // (the LM head at M <= 2), where three CUDA-core CTAs per SM stream a little faster.  QW3B200_TC_MIN_M
     // overrides: the tensor-core kernel is then used from that many activation rows upwards only.
@@ -281,9 +277,21 @@ static int gemm_dispatch(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const
         return (e && *e) ? (uint32_t)strtoul(e, nullptr, 10) : 0u;
     }();
     const bool tall_matvec = M <= 2 && w->rows_pad / 128 >= 600;
-    if (impl == 0 && M >= tc_min_m && !(tc_min_m == 0 && tall_matvec) && qb_gemm_tc_supported(w, M))
-        return qb_launch_gemm_tc(ctx, w, q, d, M, part, S);
-    return qb_launch_gemm_dp4a(ctx, w, q, d, M, part, S);
+    return impl == 0 && M >= tc_min_m && !(tc_min_m == 0 && tall_matvec) && qb_gemm_tc_supported(w, M);
+}
+
+static int gemm_dispatch(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const float *d, uint32_t M, float *part,
+                         uint32_t S, int impl, const QbGemmWork &work) {
+    if (!takes_tc(w, M, impl)) return qb_launch_gemm_dp4a(ctx, w, q, d, M, part, S);
+    if (!qb_gemm_tc_supported(w, M))
+        return qb_fail(QB_ERR_UNSUPPORTED, "tensor-core GEMM does not support this shape");
+    return qb_launch_gemm_tc(ctx, w, q, d, M, part, S, nullptr, nullptr, nullptr, work);
+}
+
+size_t qb_gemm_work_bytes(qb_ctx *ctx, const qb_weight *w, uint32_t M, uint32_t S, int impl) {
+    const size_t bytes = (size_t)M * w->cols * 2;
+    const bool used = bytes <= QB_GEMM_WORK_MAX && S > 0 && takes_tc(w, M, impl) && qb_gemm_tc_supported(w, M) && qb_gemm_f16_wins(w, M, S, (uint32_t)ctx->sm_count);
+    return used ? bytes : 0;
 }
 
 extern "C" int qb_q8_gemm_partials(qb_ctx *ctx, const qb_weight *w, const int8_t *q_dev, const float *d_dev, uint32_t M,
@@ -301,15 +309,20 @@ extern "C" int qb_q8_0_matmul(qb_ctx *ctx, const qb_weight *w, const float *x_de
     const uint32_t K = w->cols, N = w->rows, ld = qb_act_ld(M);
     const size_t qbytes = ((size_t)M * K + 255) & ~(size_t)255;
     const size_t dbytes = (((size_t)(K / 32) * ld * 4) + 255) & ~(size_t)255;
-    const size_t pbytes = (size_t)S * M * N * 4;
+    const size_t pbytes = ((size_t)S * M * N * 4 + 255) & ~(size_t)255;
+    const bool direct = S == 1 && y_stride == N;                    // a single segment is written straight to y, the partials' place is free
+    const size_t wbytes = qb_gemm_work_bytes(ctx, w, M, S, impl), in_part = direct && wbytes <= pbytes ? wbytes : 0;
     void *scr = nullptr;
-    QB_TRY(qb_ctx_scratch(ctx, qbytes + dbytes + pbytes, &scr));
+    bool extra = false;
+    QB_TRY(qb_ctx_scratch_extra(ctx, qbytes + dbytes + pbytes, wbytes - in_part, &scr, &extra));
     int8_t *q = (int8_t *)scr;
     float *d = (float *)((uint8_t *)scr + qbytes);
     float *part = (float *)((uint8_t *)scr + qbytes + dbytes);
+    QbGemmWork work;
+    if (in_part || extra) { work.p = (uint8_t *)part + (in_part ? 0 : pbytes); work.bytes = wbytes; }
     QB_TRY(qb_quantize_act(ctx, x_dev, M, K, x_stride, q, d));
-    if (S == 1 && y_stride == N) return qb_launch_gemm(ctx, w, q, d, M, y_dev, 1, impl);
-    QB_TRY(qb_launch_gemm(ctx, w, q, d, M, part, S, impl));
+    if (direct) return qb_launch_gemm(ctx, w, q, d, M, y_dev, 1, impl, work);
+    QB_TRY(qb_launch_gemm(ctx, w, q, d, M, part, S, impl, work));
     return qb_launch_reduce_parts(ctx, part, S, M, N, y_dev, y_stride);
 }
 

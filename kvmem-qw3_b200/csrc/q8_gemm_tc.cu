@@ -568,7 +568,7 @@ bool qb_gemm_tc_supported(const qb_weight *w, uint32_t M) {
 }
 
 int qb_launch_gemm_tc(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const float *d, uint32_t M, float *part, uint32_t S,
-                      const QbGemmPush *push, uint32_t *grid_out, const QbGemmSwiglu *swiglu) {
+                      const QbGemmPush *push, uint32_t *grid_out, const QbGemmSwiglu *swiglu, const QbGemmWork &work) {
     QB_REQUIRE(!swiglu || (M <= 16 && S == 1 && w->rows % 128 == 0 && w->cols / 128 > 8 && swiglu->q && swiglu->d),
                "gemm: the fused SwiGLU needs M <= 16, one K segment, whole 128-row tiles and K > 1024");
     QB_REQUIRE(M > 0 && S > 0 && S <= w->cols / 128, "gemm: bad M=%u or ksplit=%u", M, S);
@@ -579,11 +579,8 @@ int qb_launch_gemm_tc(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const fl
     if (M <= 32) return launch_tc<32, 32>(ctx, w, q, d, M, part, S, push, grid_out, swiglu);
     if (M <= 48) return launch_tc<48, 48>(ctx, w, q, d, M, part, S, push, grid_out, swiglu);
     if (M <= 64) return launch_tc<64, 64>(ctx, w, q, d, M, part, S, push, grid_out, swiglu);
-    if (!push && qb_gemm_f16_wins(w, M, S, (uint32_t)ctx->sm_count)) {
-        void *work = nullptr;
-        if (qb_ctx_scratch4(ctx, (size_t)M * w->cols * 2, &work) == QB_OK) return qb_launch_gemm_f16(ctx, w, q, d, M, work, part, S, grid_out);
-        cudaGetLastError();                                               // no room on the device: the int8 form, the same bits
-    }
+    if (!push && work.bytes >= (size_t)M * w->cols * 2 && ((uintptr_t)work.p & 15) == 0 && qb_gemm_f16_wins(w, M, S, (uint32_t)ctx->sm_count))
+        return qb_launch_gemm_f16(ctx, w, q, d, M, work.p, part, S, grid_out);
     // From 65 rows on the tile is as wide as the rows divide evenly over as few tiles as 128 columns allow, in steps of 16 (331 rows: three tiles of
     // 112): every column of a tile costs drain time, whether it holds a row or not.  34816 x 5120, tiles of 128 / as wide as needed: 65 rows 123 / 100
     // us, 100 rows 125 / 115, 160 rows 232 / 187, 331 rows 343 / 313.  For the same reason 48 columns between 32 and 64 (48 rows 70 / 65.5 us).

@@ -100,13 +100,13 @@ struct qb_ctx {
     size_t scratch2_bytes = 0;
     void *scratch3 = nullptr;              // workspace of the DeltaNet ingestion launches when the caller brings none
     size_t scratch3_bytes = 0;
-    void *scratch4 = nullptr;              // int8 activations of a many-row product as fp16
-    size_t scratch4_bytes = 0;
+    size_t scratch_denied = 0;             // bytes that the device had no room for (qb_ctx_scratch_extra), 0: none; and what was free then
+    size_t scratch_denied_free = 0;
 };
 int qb_ctx_scratch(qb_ctx *ctx, size_t bytes, void **out);
 int qb_ctx_scratch2(qb_ctx *ctx, size_t bytes, void **out);
 int qb_ctx_scratch3(qb_ctx *ctx, size_t bytes, void **out);
-int qb_ctx_scratch4(qb_ctx *ctx, size_t bytes, void **out);
+int qb_ctx_scratch_extra(qb_ctx *ctx, size_t bytes, size_t extra, void **out, bool *has_extra);
 void qb_trace_mark(qb_ctx *ctx, const char *name);
 uint32_t qb_env_u32(const char *name, uint32_t dflt);
 // Device timeline (qb_debug_timeline_*): while enabled every tensor-core GEMM launch gets a slot of
@@ -229,9 +229,15 @@ int qb_launch_swiglu_quant(qb_ctx *ctx, const float *gu, uint32_t gu_stride, uin
                            uint32_t q_pitch, float *d, uint32_t d_ld, uint32_t S = 1, size_t pstride = 0, uint32_t ileave = 0);
 
 // ---- GEMM ----------------------------------------------------------------------------------
+// Device memory that its caller has no other use for until the product is done: products of many rows take their faster form where it holds
+// M * cols * 2 bytes (the activations as fp16) and the int8 form, the same bits, where it does not.  A product allocates nothing.
+struct QbGemmWork {
+    void *p = nullptr;
+    size_t bytes = 0;
+};
 // part[s][m][n] for s < S; activations q [M][K] pitch K, d [K/32][ld].
 int qb_launch_gemm(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const float *d, uint32_t M, float *part,
-                   uint32_t S, int impl);
+                   uint32_t S, int impl, const QbGemmWork &work = QbGemmWork());
 int qb_launch_gemm_dp4a(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const float *d, uint32_t M, float *part,
                         uint32_t S);
 // Optional fan-out of the tensor-core GEMM's epilogue for the tensor-parallel FFN: every partial sum goes to
@@ -252,8 +258,11 @@ struct QbGemmSwiglu {
 };
 int qb_launch_gemm_tc(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const float *d, uint32_t M, float *part,
                       uint32_t S, const QbGemmPush *push = nullptr, uint32_t *grid_out = nullptr,
-                      const QbGemmSwiglu *swiglu = nullptr);
+                      const QbGemmSwiglu *swiglu = nullptr, const QbGemmWork &work = QbGemmWork());
 bool qb_gemm_tc_supported(const qb_weight *w, uint32_t M);
+// Work area that a product of M rows is faster with, in bytes; 0: none, or more than a call keeps for it in its context (QB_GEMM_WORK_MAX).
+constexpr size_t QB_GEMM_WORK_MAX = (size_t)128 << 20;
+size_t qb_gemm_work_bytes(qb_ctx *ctx, const qb_weight *w, uint32_t M, uint32_t S, int impl);
 // The same product with fp16 operands (q8_gemm_f16.cu, the same bits): whether it is the faster form, and its launch; work: M * cols * 2 bytes.
 bool qb_gemm_f16_wins(const qb_weight *w, uint32_t M, uint32_t S, uint32_t sms);
 int qb_launch_gemm_f16(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const float *d, uint32_t M, void *work, float *part, uint32_t S,
@@ -262,7 +271,7 @@ int qb_launch_gemm_f16(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const f
 // segment: one launch (the GEMM epilogue does it); otherwise GEMM (into act, or split partials into parts) and the
 // SwiGLU kernel.  mode: 0 = as described, 1 = always two launches, 2 = one launch or fail.
 int qb_ffn_gate_up_swiglu(qb_ctx *ctx, const qb_weight *w, const int8_t *xq, const float *xd, uint32_t M, float *act, float *parts,
-                          size_t parts_floats, int8_t *hq, uint32_t hq_pitch, float *hd, uint32_t hd_ld, int gemm_impl, int mode);
+                          size_t parts_floats, int8_t *hq, uint32_t hq_pitch, float *hd, uint32_t hd_ld, int gemm_impl, int mode, const QbGemmWork &work = QbGemmWork());
 uint32_t qb_ksplit(uint32_t N, uint32_t K);
 // Row order of a tensor-parallel group's gate/up shards: 0 = [gate; up] (the op-level entry points), 64 = the model's
 // interleaved order.

@@ -139,7 +139,9 @@ extern "C" int qb_tp_ffn_push(qb_ctx *ctx, qb_tp_group *g, const qb_weight *gate
     a.q = g->xq; a.q_pitch = g->n_in; a.d = g->xd; a.d_ld = ld;
     QB_TRY(qb_launch_norm_quant(ctx, a));
     const uint32_t S_gu = qb_ksplit(gate_up->rows, gate_up->cols);
-    QB_TRY(qb_launch_gemm(ctx, gate_up, g->xq, g->xd, M, g->gu_parts, S_gu, 0));
+    // each product's partials area is idle while the other one runs
+    QbGemmWork in_dn{g->dn_parts, g->region_floats * sizeof(float)}, in_gu{g->gu_parts, (size_t)S_gu * g->max_rows * 2 * g->f_shard * sizeof(float)};
+    QB_TRY(qb_launch_gemm(ctx, gate_up, g->xq, g->xd, M, g->gu_parts, S_gu, 0, in_dn));
     QB_TRY(qb_launch_swiglu_quant(ctx, g->gu_parts, 2 * g->f_shard, M, g->f_shard, g->hq, g->f_shard, g->hd, ld, S_gu,
                                   (size_t)M * 2 * g->f_shard, g->gu_ileave));
     const uint32_t par = g->step & 1;
@@ -154,7 +156,7 @@ extern "C" int qb_tp_ffn_push(qb_ctx *ctx, qb_tp_group *g, const qb_weight *gate
         QB_TRY(qb_launch_gemm_tc(ctx, down, g->hq, g->hd, M, nullptr, g->S_dn, &push, &grid));
         g->pushed_S[par] = g->S_dn;
     } else {
-        QB_TRY(qb_launch_gemm_tc(ctx, down, g->hq, g->hd, M, g->dn_parts, g->S_dn));
+        QB_TRY(qb_launch_gemm_tc(ctx, down, g->hq, g->hd, M, g->dn_parts, g->S_dn, nullptr, nullptr, nullptr, in_gu));
         dim3 rg((g->n_out + 255) / 256, M);
         QB_CUDA(qb_launch_pdl(ctx->stream, tp_local_reduce_push_kernel, rg, dim3(256), (size_t)0, (const float *)g->dn_parts, g->S_dn, M,
                               g->n_out, push));
