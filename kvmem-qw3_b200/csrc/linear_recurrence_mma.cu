@@ -367,7 +367,7 @@ int launch(qb_ctx *ctx, const QbRecurrence &a) {
     if constexpr (ND == 1) {
         const uint32_t heads = a.H * a.ns, sms = (uint32_t)ctx->sm_count;
         const uint32_t w32 = ((a.vdim + 31) / 32 * heads + sms - 1) / sms, w48 = ((a.vdim + 47) / 48 * heads + sms - 1) / sms;
-        if (12 * w32 > 13 * w48) return launch_width<GATED, ND, 48>(ctx, a);
+        if (100 * w32 > 109 * w48) return launch_width<GATED, ND, 48>(ctx, a);
     }
     return launch_width<GATED, ND, 32>(ctx, a);
 }

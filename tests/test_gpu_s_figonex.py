@@ -250,6 +250,38 @@ def test_recurrence_of_many_heads(make, heads, dim, vdim, gated):
     b.close()
 
 
+@pytest.mark.parametrize("gated", [False, True])
+def test_recurrence_bits_do_not_depend_on_the_slice(make, qb, ctx, gated):
+    """20 heads alone (slices of 32 value columns) and among 80 (slices of 48), the other 60 with weights of zero: the same logits, bit for bit, in
+    prompt portions and in the steps behind them.  Every projection row picks one input, and four times the heads with next to no eps scale
+    the lightning layer's norm by a power of two, so nothing but the slice's own sums can differ."""
+    dim, vdim, few, many = 24, 100, 20, 80
+    waves = lambda w, heads: -(-(-(-vdim // w) * heads) // qb.lib().qb_sm_count(ctx.h))
+    assert 100 * waves(32, many) > 109 * waves(48, many) and 100 * waves(32, few) <= 109 * waves(48, few)
+
+    def of_heads(heads):
+        decay = np.concatenate([np.linspace(0.8, 0.999, few), np.full(heads - few, 0.9)]).tolist()
+        return config([mls(heads=heads, dim=dim, vdim=vdim) if gated else lig(heads=heads, dim=dim, vdim=vdim, decay=decay)], eps=1e-30)
+
+    base, rng = F.random_weights(of_heads(few), 3), np.random.default_rng(4)
+    for name, a in base.items():
+        if name.startswith("l0.mix.") and a.ndim == 2:
+            base[name] = np.zeros_like(a)
+            base[name][np.arange(len(a)), rng.integers(0, a.shape[1], len(a))] = 1.0
+
+    def edit(W):
+        for name, a in base.items():
+            W[name][...] = 0.0
+            W[name][tuple(slice(n) for n in a.shape)] = a
+
+    toks, got = rng.integers(0, 210, 221).tolist(), []
+    for heads in (few, many):
+        b = make(of_heads(heads), edit=edit).batch("bfloat16")
+        got.append(in_portions(b, 0, toks, [150, 1, 3, 66, 1]))
+        b.close()
+    assert np.isfinite(got[0]).all() and got[0].std() > 0.1 and np.array_equal(got[0], got[1])
+
+
 def test_engine_chunks(make, monkeypatch):
     """A portion longer than the executor's own chunk, cut inside it."""
     monkeypatch.setenv("QW3B200_PREFILL_CHUNK", "48")
