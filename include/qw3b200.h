@@ -163,7 +163,8 @@ int qb_weight_q8_0_gate_up(qb_ctx *ctx, const void *gate_blocks, const void *up_
 /* q8_0_matmul_silu_mul (include/qw3/device_backend.hpp:300-539): h = silu(W_gate x) * (W_up x) for M rows, left as
  * the quantised input of the down projection: hq_dev = int8 [M][n_ff], hd_dev = float [n_ff/32][ld] (qb_quantize_act
  * layout).  With M <= 16 and a one-segment weight the GEMM's epilogue does it in one launch; otherwise GEMM + a
- * SwiGLU kernel.  mode: 0 = choose, 1 = always two launches, 2 = one launch or fail; all give the same bits. */
+ * SwiGLU kernel.  mode: 0 = choose, 1 = always two launches, 2 = one launch or fail; all give the same bits.
+ * Its work area is that of qb_q8_0_matmul. */
 int qb_q8_0_matmul_silu_mul_q8(qb_ctx *ctx, const qb_weight *gate_up, const float *x_dev, uint32_t M, uint32_t x_stride,
                                int8_t *hq_dev, float *hd_dev, int mode);
 

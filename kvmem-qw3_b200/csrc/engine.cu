@@ -381,7 +381,7 @@ static void attention_form(qb_batch *b) {
 }
 
 // Rows of a qwen35 prompt pass: 512, doubled up to 2048 while the context has use for them (fewer half-empty waves of GEMM tiles and
-// fewer launches: 2048 tokens of the 27B shape in passes of 512 / 1024 / 2048: 391 / 378 / 372 ms) and the split partials of attention
+// fewer launches: 2048 tokens of the 27B shape in passes of 512 / 1024 / 2048: 307 / 297 / 284 ms) and the split partials of attention
 // (rows x splits x heads x head size floats) stay below what 512 rows take at a context of 32768 in 256-key splits, with a few splits to
 // spare: 1.7 GB on that shape.  The other buffers of a row are 0.4 MB there (a pass of 2048 rows: 0.8 GB, of 512: 0.2).  A shard keeps 512:
 // its peers' receive areas are made for it.

@@ -6,14 +6,15 @@
 //
 // What bounds it: one multiplication (d_w*d_x) and one fma per (row, column, block) on the fp32 pipe, 128 a clock and SM: 512 cycles per
 // 128 x 256 x 32 block, which takes about 1080.  In the int8 form the conversion of every dot to fp32 takes a third of the issue slots and half
-// of another pipe's rate beside that (1440 cycles).  34816 x 5120, 512 / 2048 rows: 447 / 1645 us in int8 form, 388 / 1412 here.
+// of another pipe's rate beside that (1160 cycles).  34816 x 5120 from a cold L2, 512 / 2048 rows: 431 / 1564 us in int8 form, 400 / 1455 here with
+// the widening launch.
 //
 // Shape: 128 weight rows (MMA M) x 256 activation rows (MMA N) per CTA.  Twelve warps: warp 0 requests copies, warp 1 issues the MMAs,
 // warps 2-3 widen a stage's int8 weights to fp16 in shared memory, warps 4-11 drain, each 32 rows x 128 columns of a block (224 registers by
 // setmaxnreg: short of them the compiler copies registers around).  A stage is 64 k (two blocks): fp16 weights in a ring of their own,
 // activations (widened once per launch into a workspace by act_widen_kernel) and both scales in another.  Tensor memory holds two blocks, the
-// even and the odd one of a stage.  A stage's two blocks are straight lines of code with constant addresses (in a loop over blocks 1469 us at
-// 2048 rows), and a drain warp tests the next block's barrier before it rescales the last columns of the one at hand (without 1535).
+// even and the odd one of a stage.  A stage's two blocks are straight lines of code with constant addresses (in a loop over blocks 4 percent
+// more at 2048 rows), and a drain warp tests the next block's barrier before it rescales the last columns of the one at hand (without, in that loop, 3 more).
 // Every wait is bounded; when one runs out the CTA raises the context's error flag, lets its copies land, frees its tensor memory and returns.
 #include "qb_internal.h"
 #include "tc_common.cuh"

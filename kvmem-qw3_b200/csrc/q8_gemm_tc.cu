@@ -15,7 +15,7 @@
 // activation-row count reaches the hundreds.
 //
 // Warp roles: warp 0 = TMA producer, warp 1 = MMA issuer (owns the TMEM allocation), warps 2.. = epilogue
-// (TMEM lane quarter = warp % 4; four warps for the small tiles, eight from 32 activation rows on).  Every wait is bounded: when a wait runs out
+// (TMEM lane quarter = warp % 4; 4, 8, 12 or 16 warps by tile).  Every wait is bounded: when a wait runs out
 // the CTA raises the context's error flag, lets its copies land, frees its TMEM and returns.
 #include "qb_internal.h"
 #include "tc_common.cuh"
@@ -72,8 +72,8 @@ struct TcCfg {
     static constexpr int CTAS_PER_SM = MT == 16 ? 2 : 1;
     // Second launch bound.  Left unspecified, the compiler keeps several variants at 64 registers with spills inside
     // the drain loop (it assumes more resident CTAs than the shared memory allows); told the real residency it uses
-    // 94-168 registers, with 12 bytes of spill stores left in the 128-row variant and 106 in the 16-column one.  The 32-column
-    // variant measured faster with the default, so it keeps it (0).
+    // 90-168 registers, with 106 bytes of spill stores left in the 16-column one and none in the others.  The 32-column
+    // variant measured faster with the default (64 registers, 4 bytes of spill stores), so it keeps it (0).
     static constexpr int MIN_CTAS = MT == 32 ? 0 : CTAS_PER_SM;
     static constexpr int NSLOT = 512 / CTAS_PER_SM / (KPS * MT);
     static constexpr int TMEM_COLS = 512 / CTAS_PER_SM;
@@ -93,8 +93,8 @@ struct TcCfg {
     // The producer and issuer threads are elected (steps of 1 to 4 requests take 1 to 4 percent less than with lane 0), except in the
     // form for 5 to 8 rows, where lane 0 is the faster one (steps of 5 to 8 requests of eight 27B layers: 0.5 to 1.2 percent less).
     static constexpr bool ELECT = NLD != 8;
-    // Epilogue warps: four for the small tiles (one per TMEM lane quarter), eight or sixteen for the larger ones (two / four per
-    // quarter, each taking a slice of the activation columns).
+    // Epilogue warps: four for tiles of 16 rows (one per TMEM lane quarter), twelve at 48 rows, sixteen at 64 and eight at the others
+    // (three / four / two per quarter, each taking a slice of the activation columns).
     static constexpr int EPI_WARPS = MT == 64 ? 16 : MT == 48 ? 12 : MT >= 32 ? 8 : 4;
     static constexpr int THREADS = 64 + 32 * EPI_WARPS;
     static constexpr int NC = NLD / (EPI_WARPS / 4);             // accumulator columns per epilogue thread
@@ -346,8 +346,10 @@ gemm_tc_kernel(const uint8_t *__restrict__ rec, const __grid_constant__ CUtensor
                 // of 32 a tile of 128 takes 1.15 times as long, at 64 rows and below there is no gain.  A slot is one straight line of code: the
                 // compiler then starts the next chunk's loads before it rescales the one at hand, which branches that skip the columns beyond the
                 // last row prevent (34816 x 5120 with 128 rows 125 us, with such branches 163).
-                // But at 112 rows a warp tests the next slot's barrier before it rescales the last columns of the one at hand and a stage's slots are unrolled
-                // (34816 x 5120, 70 / 96 / 128 rows: 100 / 117 / 127 us without, 93 / 102 / 121 with; 331 rows in tiles of 112: 313 and 317.5).
+                // A warp tests the next slot's barrier before it rescales the last columns of the one at hand, and a stage's slots are unrolled (34816 x 5120,
+                // 70 / 96 / 128 rows: 100 / 117 / 127 us without, 93 / 102 / 121 with).  Not at 112 rows: there it gives tall weights 1 to 2 percent
+                // (34816 x 5120 with 331 rows 316.4 / 312.3) and costs short K segments 2 to 6 (4096 x 4096 in eight of 512, 331 rows: 52.3 / 54.3;
+                // 12288 x 2048 in three, 224 rows: 46.1 / 48.1).
                 constexpr int NC = C::NC;
                 constexpr bool AHEAD = MT != 112;
                 bool ready = false;
@@ -366,7 +368,9 @@ gemm_tc_kernel(const uint8_t *__restrict__ rec, const __grid_constant__ CUtensor
                     for (int sp = 0; sp < C::SPS; ++sp, ++j) {
                         const uint32_t slot = AHEAD && NSLOT == C::SPS ? (uint32_t)sp : j % NSLOT, sph = (j / NSLOT) & 1;
                         if constexpr (AHEAD) {
-                            // (a lane's own test may have come too early; the outcome is the warp's)
+                            // (a lane's own test may have come too early; the outcome is the warp's.  No way out on a failed wait, which would break the straight
+                            // line: to the end of the stage the warp reads tensor memory that is allocated and shared memory that is its own, the
+                            // abort flag lets every other wait fail at once, and nothing is stored once ok is false.)
                             const bool full = ready || mbar_wait(bar_tfull + 8 * slot, sph, abort_flag);
                             ok = __all_sync(0xffffffffu, full) && ok;
                         } else if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * slot, sph, abort_flag))) { ok = false; break; }
@@ -582,8 +586,9 @@ int qb_launch_gemm_tc(qb_ctx *ctx, const qb_weight *w, const int8_t *q, const fl
     if (!push && work.bytes >= (size_t)M * w->cols * 2 && ((uintptr_t)work.p & 15) == 0 && qb_gemm_f16_wins(w, M, S, (uint32_t)ctx->sm_count))
         return qb_launch_gemm_f16(ctx, w, q, d, M, work.p, part, S, grid_out);
     // From 65 rows on the tile is as wide as the rows divide evenly over as few tiles as 128 columns allow, in steps of 16 (331 rows: three tiles of
-    // 112): every column of a tile costs drain time, whether it holds a row or not.  34816 x 5120, tiles of 128 / as wide as needed: 65 rows 123 / 100
-    // us, 100 rows 125 / 115, 160 rows 232 / 187, 331 rows 343 / 313.  For the same reason 48 columns between 32 and 64 (48 rows 70 / 65.5 us).
+    // 112): every column of a tile costs drain time, whether it holds a row or not.  34816 x 5120 from a cold L2, tiles of 128 / as wide as needed,
+    // neither with the next slot tested ahead: 65 rows 123 / 100 us, 100 rows 125 / 115, 160 rows 232 / 187, 331 rows 343 / 313 (now 90, 114, 169, 316).
+    // For the same reason 48 columns between 32 and 64 (48 rows 70 / 65.5 us).
     const uint32_t m_tiles = (M + 127) / 128, width = ((M + m_tiles - 1) / m_tiles + 15) / 16 * 16;
     if (width == 80) return launch_tc<80, 80>(ctx, w, q, d, M, part, S, push, grid_out, swiglu);
     if (width == 96) return launch_tc<96, 96>(ctx, w, q, d, M, part, S, push, grid_out, swiglu);

@@ -100,9 +100,10 @@ def test_gemm_bit_exact_vs_oracle(qb, orc, ctx, N, K, M, ksplit, impl):
 
 
 @pytest.mark.parametrize("N,K,M,ksplit", [(256, 512, 16, 0), (384, 1024, 33, 2), (128, 2048, 64, 1), (640, 512, 128, 0),
-                                          (256, 640, 130, 3), (130, 256, 300, 0), (5120, 5120, 12, 0)])
+                                          (256, 640, 130, 3), (130, 256, 300, 0), (5120, 5120, 12, 0), (384, 1024, 20, 2),
+                                          (384, 1024, 90, 2)])
 def test_gemm_tensor_core_bit_exact_large_m(qb, orc, ctx, N, K, M, ksplit):
-    """tcgen05 kernel over every activation-tile width (16/32/64/128) and several tiles."""
+    """tcgen05 kernel over every activation-tile width (16/32/48/64/80/96/112/128) and several tiles."""
     rng = np.random.default_rng(N * 3 + K + M)
     blocks = _w(orc, rng, N, K)
     w = qb.Weight.from_blocks(ctx, blocks, N, K)

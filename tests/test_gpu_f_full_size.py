@@ -29,10 +29,12 @@ def test_full_size_gemm_kernels_agree_and_rows_are_batch_invariant(qb, ctx, N, K
     assert np.array_equal(tc4, _partials(qb, ctx, w, x[:4], S, 1)), "tensor-core and CUDA-core kernels differ"
     tc1 = _partials(qb, ctx, w, x[:1], S, 2)
     assert np.array_equal(tc1[:, 0], tc4[:, 0]), "row 0 alone differs from row 0 of a 4-row launch"
-    tc128 = _partials(qb, ctx, w, x, S, 2)                       # the 128-row tile, 16 epilogue warps
+    tc128 = _partials(qb, ctx, w, x, S, 2)                       # the 128-row tile
     assert np.array_equal(tc128[:, :4], tc4), "rows of a 128-row launch differ from the 4-row launch"
-    tc33 = _partials(qb, ctx, w, x[:33], S, 2)                    # 64-row tile with a ragged edge
+    tc33 = _partials(qb, ctx, w, x[:33], S, 2)                    # 48-row tile with a ragged edge
     assert np.array_equal(tc33, tc128[:, :33])
+    tc61 = _partials(qb, ctx, w, x[:61], S, 2)                    # 64-row tile with a ragged edge
+    assert np.array_equal(tc61, tc128[:, :61])
     # the split partials add up to the single-segment product (fp32 reassociation only)
     one = _partials(qb, ctx, w, x[:4], 1, 2)[0]
     tot = tc4.sum(axis=0, dtype=np.float64)
