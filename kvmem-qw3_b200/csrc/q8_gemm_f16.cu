@@ -327,8 +327,8 @@ constexpr size_t MAP_CACHE_MAX = 4096;
 // Waves of units over the SMs times a unit's time, in us for 5120 columns: 100 of this form, its share of the widening launch included; of the int8 form
 // 33 and 0.17 for each of its tile's rows (fitted to 34816 x 5120: 97 to 104 and 52 to 56).  What counts is their ratio: this form wins
 // where it needs 1 / 1.83 of the waves that tiles of 128 rows need, 1 / 1.92 of those of 112.  Over nine weights of the 27B shape and of widths
-// 2048 and 4096 at 16 row counts from 256 to 2048 the choice is within 2 percent of the faster form in 142 cases of 144 and within 3.3 in all
-// (profiles/q8_many_rows_both_forms.md).  34816 x 5120, int8 / this form: 256 rows 224 / 208 us, 330 rows 316 / 398, 512 rows 431 / 400, 640
+// 2048 and 4096 at 16 row counts from 256 to 2048 the choice is within 2 percent of the faster form in 142 cases of 144 and within 3.3 in all.
+// 34816 x 5120, int8 / this form: 256 rows 224 / 208 us, 330 rows 316 / 398, 512 rows 431 / 400, 640
 // rows 533 / 591, 1000 rows 794 / 783, 2048 rows 1564 / 1455.
 // Segments of fewer than four records keep the int8 form, which is one launch and fills its pipeline sooner.
 bool qb_gemm_f16_wins(const qb_weight *w, uint32_t M, uint32_t S, uint32_t sms) {
